@@ -36,18 +36,16 @@ namespace cbs {
 //     holds the full spectrum of output h and inverse-transforms it into registers;
 //  4. output h is staged in this half's FFT buffer and each thread updates the accumulator
 //     positions it owns: acc_h[i] += t_h[i - a] (negacyclic wrap) - t_h[i].
-template <int LOGN, bool WIDE>
+template <int LOGN>
 __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftCfg<LOGN>::MIN_BLOCKS)
     k_blind_rotate_fft(const BlindRotateArgs a, const FftKeyArgs f) {
     constexpr int LOGM = LOGN - 1;
     constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, T = 2 * TH, TWO_N = 2 * N;
     using Tb = FftTab<LOGM>;
-    using DigT = typename DigitPair<WIDE>::T;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* acc = smem;                                           // [2][N]
     double2* fs = reinterpret_cast<double2*>(smem + 2 * N);         // [2][M]
     double2* tab = fs + 2 * M;                                      // FftTab<LOGM>
-    DigT* dig = reinterpret_cast<DigT*>(tab + Tb::size());          // [2][digits][M] digit pairs
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -90,38 +88,23 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftCfg<LOGN>::MIN_BLOCKS)
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
     };
     const uint32_t l2 = 2 * digits;
-    const int32_t dbias = 1 << (gbits - 1);
+    const DigitBias bias(1u << (gbits - 1));
+    const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
     for (uint32_t step = 0; step < a.n; ++step) {
         const uint32_t at = special_ms_f(__ldg(arow + step), TWO_N, a.q_lwe, a.bitwidth);
-        // 1. digits of this half's polynomial.  Thread ht writes (and its first FFT pass
-        //    reads) exactly the positions ht + j*TH it owns, so no barrier is needed for dig;
-        //    the barrier after this loop orders the previous step's reads of my_fs before
-        //    the first transform writes it.
-        const uint32_t fmask = (1u << gbits) - 1u;
-        for (uint32_t e = ht; e < M; e += TH) {
-            const uint64_t wr = static_cast<uint64_t>(my_acc[e]) >> ign;
-            const uint64_t wi = static_cast<uint64_t>(my_acc[e + M]) >> ign;
-            DigT* dst = dig + h * digits * M + e;
-            // biased digit fields (digit + 2^(gbits-1))
-            for (uint32_t d = 0; d < digits; ++d)
-                dst[d * M] = DigitPair<WIDE>::pack(static_cast<uint32_t>(wr >> (gbits * d)) & fmask,
-                                                   static_cast<uint32_t>(wi >> (gbits * d)) & fmask);
-        }
-        half_bar();
-        // 2. forward transforms and products
+        // 1. per digit of this half's polynomial: forward transform and products.  Thread ht's first
+        // FFT pass reads exactly the accumulator positions ht + j*TH it updates itself, and first
+        // writes the exchange entries the previous inverse transform's last pass read.
         const double2* ek = f.bskf + static_cast<size_t>(step) * l2 * 2 * M + ht;
         double2 y0[8], y1[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) y0[j] = y1[j] = make_double2(0.0, 0.0);
         for (uint32_t d = 0; d < digits; ++d) {
-            const DigT* dsrc = dig + (h * digits + d) * M;
+            const int shift = ign + gbits * static_cast<int>(d);
             double2 x[8];
             fft_forward_to_regs<LOGM>(
-                my_fs, ht, tab,
-                [&](int j, uint32_t e) {
-                    return cmul(DigitPair<WIDE>::unpack(dsrc[e], dbias), twist_at<LOGM>(tws, j, e));
-                },
+                my_fs, ht, tab, [&](int, uint32_t e) { return offset_digit_pair<M>(my_acc, e, shift, fmask, bias); },
                 x, half_bar);
             const double2* k0 = ek + static_cast<size_t>(2 * d + h) * 2 * M;  // key row 2d + h, slot-major
             const double2* k1 = k0 + M;
@@ -242,20 +225,18 @@ struct BrFftMbCfg {
     static constexpr int MIN_BLOCKS = 1;
 };
 
-template <int LOGN, int MB, bool WIDE>
+template <int LOGN, int MB>
 __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftMbCfg<LOGN, MB>::MIN_BLOCKS)
     k_blind_rotate_fft_mb(const BlindRotateArgs a, const FftKeyArgs f) {
     constexpr int LOGM = LOGN - 1;
     constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, T = 2 * TH, TWO_N = 2 * N;
     constexpr uint32_t KS = mb_group_keys(MB);
     using Tb = FftTab<LOGM>;
-    using DigT = typename DigitPair<WIDE>::T;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* acc = smem;                                           // [2][N]
     double2* fs = reinterpret_cast<double2*>(smem + 2 * N);         // [2][M]
     double2* tab = fs + 2 * M;                                      // FftTab<LOGM>
-    DigT* dig = reinterpret_cast<DigT*>(tab + Tb::size());          // [2][digits][M] digit pairs
-    double2* cbuf = reinterpret_cast<double2*>(dig + 2 * a.digits * M);  // [step coefs][8][T] c_i per slot
+    double2* cbuf = tab + Tb::size();                               // [step coefs][8][T] c_i per slot
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -292,7 +273,8 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftMbCfg<LOGN, MB>::MIN_B
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
     };
     const uint32_t l2 = 2 * digits;
-    const int32_t dbias = 1 << (gbits - 1);
+    const DigitBias bias(1u << (gbits - 1));
+    const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
     const uint32_t groups = (a.n + MB - 1) / MB;
     const size_t kstride = static_cast<size_t>(l2) * 2 * M;  // spectra between subsets of a group
@@ -314,36 +296,20 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftMbCfg<LOGN, MB>::MIN_B
             for (int j = 0; j < 8; ++j) {
                 const uint32_t r3 = ((j & 1) << 2) | (j & 2) | ((j >> 2) & 1);
                 const uint32_t k = (at * r3) & 7u;
-                double2 w = tab[(k & 3u) * (M / 8)];
-                if (k & 4u) w = make_double2(-w.x, -w.y);
-                const double2 v = cmul(ub, w);
+                const double2 v = cmul(ub, omega8<double2>(k));
                 cbuf[(i * 8 + j) * T + tid] = make_double2(v.x - 1.0, v.y);
             }
         }
-        // 1. digits of this half's polynomial (thread-private positions, as in the one-bit form)
-        const uint32_t fmask = (1u << gbits) - 1u;
-        for (uint32_t e = ht; e < M; e += TH) {
-            const uint64_t wr = static_cast<uint64_t>(my_acc[e]) >> ign;
-            const uint64_t wi = static_cast<uint64_t>(my_acc[e + M]) >> ign;
-            DigT* dst = dig + h * digits * M + e;
-            for (uint32_t d = 0; d < digits; ++d)
-                dst[d * M] = DigitPair<WIDE>::pack(static_cast<uint32_t>(wr >> (gbits * d)) & fmask,
-                                                   static_cast<uint32_t>(wi >> (gbits * d)) & fmask);
-        }
-        half_bar();
-        // 2. forward transforms; per slot the combined key of row 2d + h, both columns
+        // 1. forward transforms of the digits; per slot the combined key of row 2d + h, both columns
         const double2* gk = gkey + ht;
         double2 y0[8], y1[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) y0[j] = y1[j] = make_double2(0.0, 0.0);
         for (uint32_t d = 0; d < digits; ++d) {
-            const DigT* dsrc = dig + (h * digits + d) * M;
+            const int shift = ign + gbits * static_cast<int>(d);
             double2 x[8];
             fft_forward_to_regs<LOGM>(
-                my_fs, ht, tab,
-                [&](int j, uint32_t e) {
-                    return cmul(DigitPair<WIDE>::unpack(dsrc[e], dbias), twist_at<LOGM>(tws, j, e));
-                },
+                my_fs, ht, tab, [&](int, uint32_t e) { return offset_digit_pair<M>(my_acc, e, shift, fmask, bias); },
                 x, half_bar);
             // combined keys of row 2d + h, both columns, all 8 slots: subset by subset, the 16
             // key spectra of one subset are loaded together (16 independent loads in flight)
@@ -452,7 +418,7 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, BrFftMbCfg<LOGN, MB>::MIN_B
 // spectrum by m_S(psi) and accumulates it against the subset's key spectra of row 2d + h:
 // y_c += (x_d m_S) K_S[2d + h][c].  Same arithmetic count as forming the combined key first; the
 // two live digit spectra take the registers the combined-key accumulators held.
-template <int LOGN, int MB, bool WIDE>
+template <int LOGN, int MB>
 __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
     k_blind_rotate_fft_mb_d2(const BlindRotateArgs a, const FftKeyArgs f) {
     constexpr int LOGM = LOGN - 1;
@@ -460,13 +426,11 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
     constexpr uint32_t KS = (1u << MB) - 1u;
     constexpr uint32_t DIGITS = 2;
     using Tb = FftTab<LOGM>;
-    using DigT = typename DigitPair<WIDE>::T;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* acc = smem;                                           // [2][N]
     double2* fs = reinterpret_cast<double2*>(smem + 2 * N);         // [2 halves][2 digits][M]
     double2* tab = fs + 4 * M;                                      // FftTab<LOGM>
-    DigT* dig = reinterpret_cast<DigT*>(tab + Tb::size());          // [2][2][M] digit pairs
-    double2* cbuf = reinterpret_cast<double2*>(dig + 2 * DIGITS * M);  // [MB][8][T] c_i per slot
+    double2* cbuf = tab + Tb::size();                               // [MB][8][T] c_i per slot
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -503,11 +467,11 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
     };
     constexpr uint32_t l2 = 2 * DIGITS;
-    const int32_t dbias = 1 << (gbits - 1);
+    const DigitBias bias(1u << (gbits - 1));
+    const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
     const uint32_t groups = (a.n + MB - 1) / MB;
     constexpr size_t kstride = static_cast<size_t>(l2) * 2 * M;  // spectra between subsets of a group
-    const uint32_t fmask = (1u << gbits) - 1u;
     for (uint32_t g = 0; g < groups; ++g) {
         // c_i(psi_s) for the thread's 8 slots, as in k_blind_rotate_fft_mb
 #pragma unroll
@@ -519,33 +483,18 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
             for (int j = 0; j < 8; ++j) {
                 const uint32_t r3 = ((j & 1) << 2) | (j & 2) | ((j >> 2) & 1);
                 const uint32_t k = (at * r3) & 7u;
-                double2 w = tab[(k & 3u) * (M / 8)];
-                if (k & 4u) w = make_double2(-w.x, -w.y);
-                const double2 v = cmul(ub, w);
+                const double2 v = cmul(ub, omega8<double2>(k));
                 cbuf[(i * 8 + j) * T + tid] = make_double2(v.x - 1.0, v.y);
             }
         }
-        // 1. both digits of this half's polynomial (thread-private positions)
-        for (uint32_t e = ht; e < M; e += TH) {
-            const uint64_t wr = static_cast<uint64_t>(my_acc[e]) >> ign;
-            const uint64_t wi = static_cast<uint64_t>(my_acc[e + M]) >> ign;
-            DigT* dst = dig + h * DIGITS * M + e;
-#pragma unroll
-            for (uint32_t d = 0; d < DIGITS; ++d)
-                dst[d * M] = DigitPair<WIDE>::pack(static_cast<uint32_t>(wr >> (gbits * d)) & fmask,
-                                                   static_cast<uint32_t>(wi >> (gbits * d)) & fmask);
-        }
-        half_bar();
-        // 2. the two forward transforms in lockstep
-        const DigT* d0 = dig + (h * DIGITS) * M;
-        const DigT* d1 = d0 + M;
+        // 1. the two forward transforms in lockstep
         double2 x0[8], x1[8];
         fft_forward2_to_regs<LOGM>(
             my_fs0, my_fs1, ht, tab,
-            [&](int j, uint32_t e) { return cmul(DigitPair<WIDE>::unpack(d0[e], dbias), twist_at<LOGM>(tws, j, e)); },
-            [&](int j, uint32_t e) { return cmul(DigitPair<WIDE>::unpack(d1[e], dbias), twist_at<LOGM>(tws, j, e)); },
-            x0, x1, half_bar);
-        // 3. products with the subsets' keys, row 2d + h, both columns
+            [&](int, uint32_t e) { return offset_digit_pair<M>(my_acc, e, ign, fmask, bias); },
+            [&](int, uint32_t e) { return offset_digit_pair<M>(my_acc, e, ign + gbits, fmask, bias); }, x0, x1,
+            half_bar);
+        // 2. products with the subsets' keys, row 2d + h, both columns
         const double2* gk = f.bskf + static_cast<size_t>(g) * KS * kstride + ht;
         double2 y0[8], y1[8];
 #pragma unroll
@@ -643,7 +592,7 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
 // (146 KB at N = 2048); the final accumulator passes through the spectra area for the MV
 // split.  An odd batch's last CTA runs its second ciphertext as a copy of the first and writes
 // nothing for it.
-template <int LOGN, bool WIDE>
+template <int LOGN>
 __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     k_blind_rotate_fft_mb2_x2(const BlindRotateArgs a, const FftKeyArgs f, uint32_t batch) {
     constexpr int LOGM = LOGN - 1;
@@ -723,7 +672,7 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     const uint32_t ct_bar = 1 + c2, half_id = 3 + 2 * c2 + h;
     auto ct_sync = [ct_bar]() { asm volatile("bar.sync %0, %1;" ::"r"(ct_bar), "n"(2 * TH) : "memory"); };
     auto half_bar = [half_id]() { asm volatile("bar.sync %0, %1;" ::"r"(half_id), "n"(TH) : "memory"); };
-    const int32_t dbias = 1 << (gbits - 1);
+    const DigitBias bias(1u << (gbits - 1));
     const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow[2];
 #pragma unroll
@@ -738,8 +687,6 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     };
     const uint32_t groups = (a.n + 1) / 2;
     constexpr size_t kstride = static_cast<size_t>(L2) * 2 * M;  // spectra between subsets of a group
-    // omega8 = tab[M/8] = (w8r, w8s w8r) and omega8^2 = tab[M/4] = (0, w8s)
-    const double w8r = tab[M / 8].x, w8s = tab[2 * (M / 8)].y;
     for (uint32_t g = 0; g < groups; ++g) {
         // 1. the two digit transforms of polynomial h, digits read from the accumulator
         double2 x0[8], x1[8];
@@ -747,18 +694,15 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
             uint32_t wa[16], wb[16];
             tmem_load16(tacc, wa);
             tmem_load16(tacc + 16, wb);
-            auto digit_pair = [&](int j, uint32_t e, int shift) {
+            auto digit_pair = [&](int j, int shift) {
                 const uint32_t(&w)[16] = j < 4 ? wa : wb;
                 const uint64_t wr = static_cast<uint64_t>(unpack(w, 4 * (j & 3))) >> (ign + shift);
                 const uint64_t wi = static_cast<uint64_t>(unpack(w, 4 * (j & 3) + 2)) >> (ign + shift);
-                return cmul(DigitPair<true>::unpack(make_uint2(static_cast<uint32_t>(wr) & fmask,
-                                                               static_cast<uint32_t>(wi) & fmask),
-                                                    dbias),
-                            twist_at<LOGM>(tws, j, e));
+                return make_double2(bias(static_cast<uint32_t>(wr) & fmask), bias(static_cast<uint32_t>(wi) & fmask));
             };
             fft_forward2_to_regs<LOGM>(
-                my_s0, my_s1, ht, tab, [&](int j, uint32_t e) { return digit_pair(j, e, 0); },
-                [&](int j, uint32_t e) { return digit_pair(j, e, gbits); }, x0, x1, half_bar);
+                my_s0, my_s1, ht, tab, [&](int j, uint32_t) { return digit_pair(j, 0); },
+                [&](int j, uint32_t) { return digit_pair(j, gbits); }, x0, x1, half_bar);
         }
         half_bar();  // the transforms' last reads of my_s0 / my_s1 are done
 #pragma unroll
@@ -791,13 +735,7 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
             for (int c = 0; c < 2; ++c) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    // omega8^k from its two distinct magnitudes (no table read)
-                    const uint32_t k = (at[c][i] * r3) & 7u, k3 = k & 3u;
-                    double2 w;
-                    w.x = k3 == 0 ? 1.0 : (k3 == 2 ? 0.0 : (k3 == 1 ? w8r : -w8r));
-                    w.y = k3 == 0 ? 0.0 : (k3 == 2 ? w8s : w8s * w8r);
-                    if (k & 4u) w = make_double2(-w.x, -w.y);
-                    cc[c][i] = cmul(ub[c][i], w);
+                    cc[c][i] = cmul(ub[c][i], omega8<double2>((at[c][i] * r3) & 7u));
                     cc[c][i].x -= 1.0;
                 }
                 cc[c][2] = cmul(cc[c][0], cc[c][1]);
@@ -894,29 +832,22 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
 cudaError_t ntt_forward(uint64_t* out, const uint64_t* in, const uint64_t* tw, const uint64_t* tws,
                         const cbs_dmodulus* mod, size_t dim, size_t batch, cudaStream_t s);
 
-template <int LOGN, bool WIDE>
+template <int LOGN>
 static cudaError_t br_fft_launch(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch, cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
-    const size_t smem = 2ull * N * sizeof(uint64_t) + (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) +
-                        2ull * a.digits * M * sizeof(typename DigitPair<WIDE>::T);
+    const size_t smem = 2ull * N * sizeof(uint64_t) + (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2);
     if (f.tab_len != FftTab<LOGN - 1>::size()) return cudaErrorInvalidValue;
     static size_t configured[64] = {};  // per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft<LOGN, WIDE>,
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft<LOGN>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured[dev] = smem;
     }
-    k_blind_rotate_fft<LOGN, WIDE><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
+    k_blind_rotate_fft<LOGN><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
     return cudaGetLastError();
-}
-
-template <int LOGN>
-static cudaError_t br_fft_launch(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch, cudaStream_t s) {
-    return wide_digits(a.g.gbits) ? br_fft_launch<LOGN, true>(a, f, batch, s)
-                                  : br_fft_launch<LOGN, false>(a, f, batch, s);
 }
 
 cudaError_t launch_blind_rotate_fft(const BlindRotateArgs& a, const FftKeyArgs& f, const cbs_dmodulus* d_mod,
@@ -934,43 +865,43 @@ cudaError_t launch_blind_rotate_fft(const BlindRotateArgs& a, const FftKeyArgs& 
     return ntt_forward(a.mv_out, a.mv_out, a.t.rp, a.t.rps, d_mod, N, static_cast<size_t>(batch) * a.num_lut * 2, s);
 }
 
-template <int LOGN, int MB, bool WIDE>
-static cudaError_t br_fft_mb_launch(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch, cudaStream_t s) {
+template <int LOGN, int MB>
+static cudaError_t br_fft_mb_digitwise_launch(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch,
+                                              cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
     const size_t smem = 2ull * N * sizeof(uint64_t) + (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) +
-                        2ull * a.digits * M * sizeof(typename DigitPair<WIDE>::T) +
                         mb_step_coefs(MB) * 8ull * BrFftCfg<LOGN>::T * sizeof(double2);
     if (f.tab_len != FftTab<LOGN - 1>::size()) return cudaErrorInvalidValue;
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb<LOGN, MB, WIDE>,
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb<LOGN, MB>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured[dev] = smem;
     }
-    k_blind_rotate_fft_mb<LOGN, MB, WIDE><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
+    k_blind_rotate_fft_mb<LOGN, MB><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
     return cudaGetLastError();
 }
 
-template <int LOGN, int MB, bool WIDE>
+template <int LOGN, int MB>
 static cudaError_t br_fft_mb_d2_launch(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch,
                                        cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
     const size_t smem = 2ull * N * sizeof(uint64_t) + (4ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) +
-                        4ull * M * sizeof(typename DigitPair<WIDE>::T) + MB * 8ull * BrFftCfg<LOGN>::T * sizeof(double2);
+                        MB * 8ull * BrFftCfg<LOGN>::T * sizeof(double2);
     if (f.tab_len != FftTab<LOGN - 1>::size()) return cudaErrorInvalidValue;
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb_d2<LOGN, MB, WIDE>,
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb_d2<LOGN, MB>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured[dev] = smem;
     }
-    k_blind_rotate_fft_mb_d2<LOGN, MB, WIDE><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
+    k_blind_rotate_fft_mb_d2<LOGN, MB><<<batch, BrFftCfg<LOGN>::T, smem, s>>>(a, f);
     return cudaGetLastError();
 }
 
@@ -985,12 +916,12 @@ static cudaError_t br_fft_mb2_x2_launch(const BlindRotateArgs& a, const FftKeyAr
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb2_x2<LOGN, true>,
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_mb2_x2<LOGN>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured[dev] = smem;
     }
-    k_blind_rotate_fft_mb2_x2<LOGN, true><<<(batch + 1) / 2, 4 * (N / 16), smem, s>>>(a, f, batch);
+    k_blind_rotate_fft_mb2_x2<LOGN><<<(batch + 1) / 2, 4 * (N / 16), smem, s>>>(a, f, batch);
     return cudaGetLastError();
 }
 
@@ -1006,11 +937,9 @@ static cudaError_t br_fft_mb_launch(const BlindRotateArgs& a, const FftKeyArgs& 
         // the two-digit gadget: both digit transforms in lockstep unless the digit-by-digit
         // schedule was chosen
         if (a.digits == 2 && a.schedule != CBS_BR_SCHEDULE_DIGITWISE)
-            return wide_digits(a.g.gbits) ? br_fft_mb_d2_launch<LOGN, MB, true>(a, f, batch, s)
-                                          : br_fft_mb_d2_launch<LOGN, MB, false>(a, f, batch, s);
+            return br_fft_mb_d2_launch<LOGN, MB>(a, f, batch, s);
     }
-    return wide_digits(a.g.gbits) ? br_fft_mb_launch<LOGN, MB, true>(a, f, batch, s)
-                                  : br_fft_mb_launch<LOGN, MB, false>(a, f, batch, s);
+    return br_fft_mb_digitwise_launch<LOGN, MB>(a, f, batch, s);
 }
 
 cudaError_t launch_blind_rotate_fft_mb(const BlindRotateArgs& a, const FftKeyArgs& f, const cbs_dmodulus* d_mod,
@@ -1060,28 +989,45 @@ static void fft_tables_for(std::vector<double2>& tab) {
         const long double ang = 2.0L * pi * e / M;
         return make_double2(static_cast<double>(cosl(ang)), static_cast<double>(sinl(ang)));
     };
+    // constant of block b of forward stage st
+    auto root = [&](int st, uint32_t b) {
+        uint32_t r = 0;
+        for (int k = 0; k < st; ++k) r |= ((b >> k) & 1u) << (st - 1 - k);
+        const long double ang = pi * (4 * r + 1) / (4.0L * (1u << st));
+        return make_double2(static_cast<double>(cosl(ang)), static_cast<double>(sinl(ang)));
+    };
     tab.assign(Tb::size(), make_double2(0, 0));
-    for (uint32_t e = 0; e < M / 2; ++e) tab[e] = tw(e);
     for (int p = 1; p < Pl::P; ++p) {
-        const uint32_t m = Tb::pass_m(p), o = Tb::pass_off(p);
-        const int r = Tb::pass_r(p);
+        const uint32_t m = Tb::pass_m(p), o = Tb::fwd_off(p), T = M / 8;
+        const int r = Tb::pass_r(p), st = 3 * p;
         if (r == 3) {
-            const uint32_t q = M / (8 * m);
-            for (uint32_t j0 = 0; j0 < q; ++j0) {
-                for (uint32_t k = 0; k < 4; ++k) tab[o + k * q + j0] = tw((j0 + k * q) * m);
-                for (uint32_t k = 0; k < 2; ++k) tab[o + 4 * q + k * q + j0] = tw((j0 + k * q) * 2 * m);
-                tab[o + 6 * q + j0] = tw(j0 * 4 * m);
+            for (uint32_t k = 0; k < m; ++k) {
+                tab[o + k] = root(st, k);
+                tab[o + m + k] = root(st + 1, 2 * k);
+                tab[o + 2 * m + k] = root(st + 2, 4 * k);
+                tab[o + 3 * m + k] = root(st + 2, 4 * k + 2);
             }
         } else if (r == 2) {
-            const uint32_t q = M / (4 * m);
-            for (uint32_t j0 = 0; j0 < q; ++j0) {
-                tab[o + j0] = tw(j0 * m);
-                tab[o + q + j0] = tw((j0 + q) * m);
-                tab[o + 2 * q + j0] = tw(j0 * 2 * m);
+            for (uint32_t t = 0; t < T; ++t) {
+                tab[o + t] = root(st, 2 * t);
+                tab[o + T + t] = root(st + 1, 4 * t);
+                tab[o + 2 * T + t] = root(st + 1, 4 * t + 2);
             }
         } else {
-            const uint32_t h = M / (2 * m);
-            for (uint32_t j0 = 0; j0 < h; ++j0) tab[o + j0] = tw(j0 * m);
+            for (uint32_t t = 0; t < T; ++t) {
+                tab[o + t] = root(st, 4 * t);
+                tab[o + T + t] = root(st, 4 * t + 2);
+            }
+        }
+    }
+    for (int p = 0; p < Pl::P; ++p) {
+        if (Tb::pass_r(p) != 3) continue;
+        const uint32_t m = Tb::pass_m(p), o = Tb::inv_off(p), q = M / (8 * m);
+        for (uint32_t j0 = 0; j0 < q; ++j0) {
+            tab[o + j0] = tw(j0 * m);
+            tab[o + q + j0] = tw((j0 + q) * m);
+            tab[o + 2 * q + j0] = tw(2 * j0 * m);
+            tab[o + 3 * q + j0] = tw(4 * j0 * m);
         }
     }
     for (uint32_t e = 0; e <= M / 2; ++e) {

@@ -48,9 +48,8 @@ __device__ __forceinline__ void fft_of_poly(double2* fs, uint32_t tid, const dou
     const uint64_t qhalf = Q >> 1;
     fft_forward_to_regs<LOGM>(
         fs, tid, tab,
-        [&](int j, uint32_t e) {
-            return cmul(make_double2(centred_double(p[e], Q, qhalf), centred_double(p[e + M], Q, qhalf)),
-                        twist_at<LOGM>(tws, j, e));
+        [&](int, uint32_t e) {
+            return make_double2(centred_double(p[e], Q, qhalf), centred_double(p[e + M], Q, qhalf));
         },
         x, bar);
 }
@@ -83,9 +82,8 @@ __device__ __forceinline__ void key_switch_products(double2* fs, uint32_t tid, c
             [&](int j, uint32_t e) {
                 const int64_t wr = prep(e);
                 const int64_t wi = prep(e + M);
-                return cmul(make_double2(static_cast<double>(balanced_digit(wr, gbits, d)),
-                                         static_cast<double>(balanced_digit(wi, gbits, d))),
-                            twist_at<LOGM>(tws, j, e));
+                return make_double2(static_cast<double>(balanced_digit(wr, gbits, d)),
+                                    static_cast<double>(balanced_digit(wi, gbits, d)));
             },
             x, []() { __syncthreads(); });
         const double2* kh = key + static_cast<size_t>(d) * 3 * M + tid;
@@ -249,9 +247,8 @@ __device__ __forceinline__ void cmux_digit_fft(double2* fs, uint32_t tid, const 
         fs, tid, tab,
         [&](int j, uint32_t e) {
             const uint2 w = src[e];
-            return cmul(make_double2(static_cast<double>(balanced_digit(w.x, gbits, d)),
-                                     static_cast<double>(balanced_digit(w.y, gbits, d))),
-                        twist_at<LOGM>(tws, j, e));
+            return make_double2(static_cast<double>(balanced_digit(w.x, gbits, d)),
+                                static_cast<double>(balanced_digit(w.y, gbits, d)));
         },
         x, bar);
 }

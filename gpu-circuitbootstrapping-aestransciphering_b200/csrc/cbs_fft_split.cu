@@ -38,26 +38,24 @@ struct BrSplitCfg {
 
 // Two halves of M/8 threads per CTA (k_blind_rotate_fft's organisation).  Per step (MB = 1) or
 // group of two coefficients (MB = 2):
-//  1. digits of each half's accumulator polynomial, packed biased pairs in shared memory;
-//  2. half h forward-transforms its DIG digit polynomials into registers;
-//  3. per limb l: both key columns of rows 2d + h, limb l (MB = 2: the combined keys
+//  1. half h forward-transforms the DIG digit polynomials of its accumulator polynomial into
+//     registers;
+//  2. per limb l: both key columns of rows 2d + h, limb l (MB = 2: the combined keys
 //     c0 (K0 + c1 K01) + c1 K1, one column at a time), against the digit spectra; the halves
 //     swap partial sums so half h holds output h; MB = 1: times psi^a - 1; inverse transform;
 //     each coefficient rounds to the exact integer limb product, is scaled by 2^(lb l) mod Q and
 //     added to the accumulator position this thread owns.
-template <int LOGN, bool WIDE, int DIG, int MB>
+template <int LOGN, int DIG, int MB>
 __global__ void __launch_bounds__(BrSplitCfg<LOGN>::T, BrSplitCfg<LOGN>::MIN_BLOCKS)
     k_blind_rotate_fft_split(const BlindRotateArgs a, const FftKeyArgs f, const SplitKeyArgs sk) {
     constexpr int LOGM = LOGN - 1;
     constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, T = 2 * TH, TWO_N = 2 * N;
     using Tb = FftTab<LOGM>;
-    using DigT = typename DigitPair<WIDE>::T;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* acc = smem;                                           // [2][N]
     double2* fs = reinterpret_cast<double2*>(smem + 2 * N);         // [2][M]
     double2* tab = fs + 2 * M;                                      // FftTab<LOGM>
-    DigT* dig = reinterpret_cast<DigT*>(tab + Tb::size());          // [2][DIG][M] digit pairs
-    double2* cbuf = reinterpret_cast<double2*>(dig + 2 * DIG * M);  // MB = 2: [2][8][T] c_i per slot
+    double2* cbuf = tab + Tb::size();                               // MB = 2: [2][8][T] c_i per slot
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -104,7 +102,7 @@ __global__ void __launch_bounds__(BrSplitCfg<LOGN>::T, BrSplitCfg<LOGN>::MIN_BLO
         return static_cast<int64_t>(mul_shoup(vm, pw, pws, Q));
     };
     const uint32_t limbs = sk.limbs;
-    const int32_t dbias = 1 << (gbits - 1);
+    const DigitBias bias(1u << (gbits - 1));
     const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
     // key polynomials per step and limb: [subsets][2*DIG rows][2 columns]
@@ -131,33 +129,20 @@ __global__ void __launch_bounds__(BrSplitCfg<LOGN>::T, BrSplitCfg<LOGN>::MIN_BLO
                 }
             }
         }
-        // 1. digits of this half's polynomial (positions ht + j*TH, owned by this thread)
-        for (uint32_t e = ht; e < M; e += TH) {
-            const uint64_t wr = static_cast<uint64_t>(my_acc[e]) >> ign;
-            const uint64_t wi = static_cast<uint64_t>(my_acc[e + M]) >> ign;
-            DigT* dst = dig + h * DIG * M + e;
-#pragma unroll
-            for (int d = 0; d < DIG; ++d)
-                dst[d * M] = DigitPair<WIDE>::pack(static_cast<uint32_t>(wr >> (gbits * d)) & fmask,
-                                                   static_cast<uint32_t>(wi >> (gbits * d)) & fmask);
-        }
-        half_bar();
-        // 2. digit spectra, held for every limb
+        // 1. digit spectra, held for every limb (digits read from the accumulator positions
+        // ht + j*TH this thread owns)
         double2 x[DIG][8];
 #pragma unroll
         for (int d = 0; d < DIG; ++d) {
-            const DigT* dsrc = dig + (h * DIG + d) * M;
             fft_forward_to_regs<LOGM>(
                 my_fs, ht, tab,
-                [&](int j, uint32_t e) {
-                    return cmul(DigitPair<WIDE>::unpack(dsrc[e], dbias), twist_at<LOGM>(tws, j, e));
-                },
-                x[d], half_bar);
+                [&](int, uint32_t e) { return offset_digit_pair<M>(my_acc, e, ign + gbits * d, fmask, bias); }, x[d],
+                half_bar);
             half_bar();
         }
         const uint32_t mbase = mult_base<LOGN>(ht, at[0]);
         const double2* ek = sk.bskx + static_cast<size_t>(step) * limbs * PER_STEP * M + ht;
-        // 3. one product, swap and inverse transform per limb
+        // 2. one product, swap and inverse transform per limb
 #pragma unroll 1
         for (uint32_t l = 0; l < limbs; ++l) {
             const double2* el = ek + static_cast<size_t>(l) * PER_STEP * M;
@@ -272,40 +257,39 @@ __global__ void __launch_bounds__(BrSplitCfg<LOGN>::T, BrSplitCfg<LOGN>::MIN_BLO
 cudaError_t ntt_forward(uint64_t* out, const uint64_t* in, const uint64_t* tw, const uint64_t* tws,
                         const cbs_dmodulus* mod, size_t dim, size_t batch, cudaStream_t s);
 
-template <int LOGN, bool WIDE, int DIG, int MB>
+template <int LOGN, int DIG, int MB>
 static cudaError_t br_split_launch(const BlindRotateArgs& a, const FftKeyArgs& f, const SplitKeyArgs& k,
                                    uint32_t batch, cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2, T = BrSplitCfg<LOGN>::T;
     const size_t smem = 2ull * N * sizeof(uint64_t) + (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) +
-                        2ull * DIG * M * sizeof(typename DigitPair<WIDE>::T) +
                         (MB == 2 ? 2ull * 8 * T * sizeof(double2) : 0);
     static size_t configured[64] = {};  // per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_split<LOGN, WIDE, DIG, MB>,
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_split<LOGN, DIG, MB>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         configured[dev] = smem;
     }
-    k_blind_rotate_fft_split<LOGN, WIDE, DIG, MB><<<batch, T, smem, s>>>(a, f, k);
+    k_blind_rotate_fft_split<LOGN, DIG, MB><<<batch, T, smem, s>>>(a, f, k);
     return cudaGetLastError();
 }
 
-template <int LOGN, bool WIDE>
+template <int LOGN>
 static cudaError_t br_split_launch(const BlindRotateArgs& a, const FftKeyArgs& f, const SplitKeyArgs& k,
                                    uint32_t batch, uint32_t mb, cudaStream_t s) {
     if (mb == 2) {
         switch (a.digits) {
-            case 2: return br_split_launch<LOGN, WIDE, 2, 2>(a, f, k, batch, s);
-            case 3: return br_split_launch<LOGN, WIDE, 3, 2>(a, f, k, batch, s);
+            case 2: return br_split_launch<LOGN, 2, 2>(a, f, k, batch, s);
+            case 3: return br_split_launch<LOGN, 3, 2>(a, f, k, batch, s);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (a.digits) {
-        case 2: return br_split_launch<LOGN, WIDE, 2, 1>(a, f, k, batch, s);
-        case 3: return br_split_launch<LOGN, WIDE, 3, 1>(a, f, k, batch, s);
-        case 4: return br_split_launch<LOGN, WIDE, 4, 1>(a, f, k, batch, s);
+        case 2: return br_split_launch<LOGN, 2, 1>(a, f, k, batch, s);
+        case 3: return br_split_launch<LOGN, 3, 1>(a, f, k, batch, s);
+        case 4: return br_split_launch<LOGN, 4, 1>(a, f, k, batch, s);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -318,14 +302,13 @@ cudaError_t launch_blind_rotate_fft_split(const BlindRotateArgs& a, const FftKey
     if (mb != 1 && mb != 2) return cudaErrorInvalidValue;
     if (k.limbs < 1 || k.limbs > kMaxSplitLimbs || k.bskx == nullptr) return cudaErrorInvalidValue;
     if (f.tab_len != (N == 1024 ? FftTab<9>::size() : FftTab<10>::size())) return cudaErrorInvalidValue;
-    const bool wide = wide_digits(a.g.gbits);
     cudaError_t e;
     switch (N) {
         case 1024:
-            e = wide ? br_split_launch<10, true>(a, f, k, batch, mb, s) : br_split_launch<10, false>(a, f, k, batch, mb, s);
+            e = br_split_launch<10>(a, f, k, batch, mb, s);
             break;
         case 2048:
-            e = wide ? br_split_launch<11, true>(a, f, k, batch, mb, s) : br_split_launch<11, false>(a, f, k, batch, mb, s);
+            e = br_split_launch<11>(a, f, k, batch, mb, s);
             break;
         default: return cudaErrorInvalidValue;
     }

@@ -2,15 +2,24 @@
 // products over Z[X]/(X^N + 1) on sm_100a.
 //
 // Folding (the scheme of bitwise/src/fft.cu:3614-3755, written from the mathematics): a
-// real length-N polynomial a is evaluated at the odd powers zeta^(4k+1), zeta = e^(i*pi/N),
-// as a cyclic length-M DFT of z_j = (a_j + i*a_(j+M)) * zeta^j; products of evaluations are
-// evaluations of the negacyclic product, and the inverse DFT, the untwist by zeta^-j and the
-// unfold (real part -> c_j, imaginary part -> c_(j+M)) recover it.
-// Forward: decimation in frequency, natural order in, bit-reversed spectrum out; inverse:
-// decimation in time, bit-reversed in, natural out (no bit-reversal pass either way, the
-// spectra of keys are stored in the same bit-reversed order).  M/8 threads, eight complex
-// values per thread, three stages per shared-memory round trip; the 16-byte elements are
-// swizzled e ^ ((e >> 3) & 7), which makes every pass free of bank conflicts for M = 1024.
+// real length-N polynomial a is evaluated at the odd powers zeta^(4k+1), zeta = e^(i*pi/N):
+// with z_j = a_j + i*a_(j+M) these are the values of z(Y) = sum z_j Y^j at the M roots of
+// Y^M = i; products of evaluations are evaluations of the negacyclic product.
+// Forward: the remainder tree of Y^M - i.  A stage splits Y^(2h) - c^2 into (Y^h - c)(Y^h + c),
+// (u, v) -> (u + c v, u - c v), with one constant c per block, so no twist of the inputs is
+// needed (it is absorbed in the constants), the first pass's constants are literals and a
+// block's threads share theirs; natural order in, bit-reversed spectrum out.  u - c v is formed
+// as 2 u - (u + c v): six fused multiply-adds a butterfly, where a twisted decimation in
+// frequency takes eight operations a butterfly and four an input.  Measured beside that form
+// (same kernels, twisted inputs, four-operation complex products): 64 NAND gates 4547 -> 4125
+// us, 1731 ragged bootstraps 48.9 -> 45.3 ms, 200 exact split-FFT circuit bootstraps 18.8 ->
+// 17.9 ms, 13 AES blocks 391 -> 386 ms; no kernel slower.
+// Inverse: decimation in time, bit-reversed in, natural out, (p, s) -> (p + s conj(w),
+// p - s conj(w)) in the same six operations, then the untwist by zeta^-j by the caller (real
+// part -> c_j, imaginary part -> c_(j+M)).  No bit-reversal pass either way: the spectra of
+// keys are stored in the same bit-reversed order.  M/8 threads, eight complex values per
+// thread, three stages per shared-memory round trip; the 16-byte elements are swizzled
+// e ^ ((e >> 3) & 7), which makes every pass free of bank conflicts for M = 1024.
 // The thread/index structure is the one of the integer NTT (ntt_core.cuh): the pass that
 // starts at DFT half-size h uses the sets of the NTT pass at stage m = M / (2h).
 #pragma once
@@ -63,245 +72,222 @@ __device__ __forceinline__ uint32_t cswz_of(uint32_t e) {
     else return cswz(e);
 }
 
-// DIF butterfly: (u, v) -> (u + v, (u - v) * w)
+// component types of the complex values
+__device__ __forceinline__ double fma_of(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fma_of(float a, float b, float c) { return fmaf(a, b, c); }
 template <class C>
-__device__ __forceinline__ void dif_bf(C& u, C& v, C w) {
-    const C s = cadd(u, v);
-    v = cmul(csubd(u, v), w);
-    u = s;
+using real_of = decltype(C::x);
+
+// forward butterfly: (u, v) -> (u + c v, u - c v)
+template <class C>
+__device__ __forceinline__ void ct_bf(C& u, C& v, C c) {
+    using R = real_of<C>;
+    C p;
+    p.x = fma_of(c.x, v.x, fma_of(-c.y, v.y, u.x));
+    p.y = fma_of(c.x, v.y, fma_of(c.y, v.x, u.y));
+    v.x = fma_of(R(2), u.x, -p.x);
+    v.y = fma_of(R(2), u.y, -p.y);
+    u = p;
 }
-// DIT butterfly (inverse of the above up to a factor 2): (p, s) -> (p + s*conj(w), p - s*conj(w))
+// inverse butterfly: (p, s) -> (p + s conj(w), p - s conj(w))
 template <class C>
 __device__ __forceinline__ void dit_bf(C& p, C& s, C w) {
-    const C t = cmulc(s, w);
+    using R = real_of<C>;
+    C t;
+    t.x = fma_of(w.x, s.x, fma_of(w.y, s.y, p.x));
+    t.y = fma_of(w.x, s.y, fma_of(-w.y, s.x, p.y));
+    s.x = fma_of(R(2), p.x, -t.x);
+    s.y = fma_of(R(2), p.y, -t.y);
+    p = t;
+}
+// the inverse butterflies with w = 1 and w = i
+template <class C>
+__device__ __forceinline__ void dit_bf_one(C& p, C& s) {
+    const C t = s;
     s = csubd(p, t);
     p = cadd(p, t);
 }
+template <class C>
+__device__ __forceinline__ void dit_bf_i(C& p, C& s) {
+    C t = mul_negi(s);
+    dit_bf_one(p, t);
+    s = t;
+}
 
-// Twiddle tables of one transform length, kept in shared memory by the kernels:
-//   [0, M/2)            tw[e] = exp(2*pi*i*e/M), read directly by the first pass (its index
-//                       runs over consecutive e);
-//   pass_off(p), p >= 1 the twiddles of pass p laid out [k][j0] (k = the butterfly's place in
-//                       the pass, j0 = the thread's group), so the lanes of a warp read
-//                       consecutive entries;
-//   twist_off()         exp(i*pi*e/N) for e <= M/2 (e > M/2 uses zeta^(M-e) = i conj(zeta^e),
-//                       i.e. the swapped components of entry M - e).
+// omega8^k = exp(i pi k / 4)
+constexpr double kSqrtHalf = 0.70710678118654752440;
+template <class C>
+__device__ __forceinline__ C omega8(uint32_t k) {
+    using R = real_of<C>;
+    const R s = static_cast<R>(kSqrtHalf);
+    const uint32_t k3 = k & 3u;
+    C w;
+    w.x = k3 == 0 ? R(1) : (k3 == 2 ? R(0) : (k3 == 1 ? s : -s));
+    w.y = k3 == 0 ? R(0) : (k3 == 2 ? R(1) : s);
+    if (k & 4u) {
+        w.x = -w.x;
+        w.y = -w.y;
+    }
+    return w;
+}
+
+// Constant tables of one transform length, kept in shared memory by the kernels (indices
+// consecutive over the lanes of a warp, or shared by them):
+//   fwd_off(p), p >= 1 the block constants of forward pass p, with c(st, b) =
+//                      exp(i pi (4 rev_st(b) + 1) / (4 2^st)) the constant of block b of stage st
+//                      (c(st, b + 1) = i c(st, b) for even b).  Three stages from st = 3p, block
+//                      k: [c(st, k)] [c(st+1, 2k)] [c(st+2, 4k)] [c(st+2, 4k+2)], 8^p entries
+//                      each; a two-stage tail, thread t: [c(st, 2t)] [c(st+1, 4t)]
+//                      [c(st+1, 4t+2)], a one-stage tail: [c(st, 4t)] [c(st, 4t+2)], M/8 each;
+//   inv_off(p)         the twiddles tw(e) = exp(2 pi i e / M) of inverse pass p over three stages
+//                      of half-size up to h = M / (2 8^p), m = 8^p, q = h/4, position j0 < q:
+//                      [tw(j0 m)] [tw((j0 + q) m)] [tw(2 j0 m)] [tw(4 j0 m)] (the others are
+//                      these times i); the tail's twiddles are 1 and i;
+//   twist_off()        exp(i*pi*e/N) for e <= M/2 (e > M/2 uses zeta^(M-e) = i conj(zeta^e),
+//                      i.e. the swapped components of entry M - e).
 template <int LOGM>
 struct FftTab {
     static constexpr uint32_t M = 1u << LOGM;
     using Pl = NttPlan<LOGM>;
     static constexpr uint32_t pass_m(int p) { return 1u << (3 * p); }
     static constexpr int pass_r(int p) { return p < Pl::P - 1 ? 3 : Pl::tail_r; }
-    static constexpr uint32_t pass_size(int p) {
-        return pass_r(p) == 3 ? 7 * (M / (8 * pass_m(p)))
-                              : (pass_r(p) == 2 ? 3 * (M / (4 * pass_m(p))) : M / (2 * pass_m(p)));
+    static constexpr uint32_t fwd_size(int p) {
+        return p == 0 ? 0 : (pass_r(p) == 3 ? 4 * pass_m(p) : (pass_r(p) == 2 ? 3 * (M / 8) : 2 * (M / 8)));
     }
-    static constexpr uint32_t pass_off(int p) {
-        uint32_t o = M / 2;
-        for (int k = 1; k < p; ++k) o += pass_size(k);
+    static constexpr uint32_t inv_size(int p) { return pass_r(p) == 3 ? 4 * (M / (8 * pass_m(p))) : 0; }
+    static constexpr uint32_t fwd_off(int p) {
+        uint32_t o = 0;
+        for (int k = 1; k < p; ++k) o += fwd_size(k);
         return o;
     }
-    static constexpr uint32_t twist_off() { return pass_off(Pl::P); }
+    static constexpr uint32_t inv_off(int p) {
+        uint32_t o = fwd_off(Pl::P);
+        for (int k = 0; k < p; ++k) o += inv_size(k);
+        return o;
+    }
+    static constexpr uint32_t twist_off() { return inv_off(Pl::P); }
     static constexpr uint32_t size() { return twist_off() + M / 2 + 1; }
 };
 
-// DIF pass over R stages starting at DFT half-size h = M / (2m).  COMPACT: tb is the pass's
-// [k][j0] table; otherwise tb is tw, indexed directly.  Twiddles known to be 1 or i are
-// applied without multiplications.
-template <int LOGM, int R, bool COMPACT, class C>
-__device__ __forceinline__ void dif_pass(C (&x)[8], uint32_t m, uint32_t tid, const C* tb) {
+// three forward stages: block constants c0 of the first stage, c1 and i c1 of the second, c2,
+// i c2, c3 and i c3 of the third
+template <class C>
+__device__ __forceinline__ void fwd_stages3(C (&x)[8], C c0, C c1, C c2, C c3) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) ct_bf(x[r], x[r + 4], c0);
+    ct_bf(x[0], x[2], c1);
+    ct_bf(x[1], x[3], c1);
+    ct_bf(x[4], x[6], mul_i(c1));
+    ct_bf(x[5], x[7], mul_i(c1));
+    ct_bf(x[0], x[1], c2);
+    ct_bf(x[2], x[3], mul_i(c2));
+    ct_bf(x[4], x[5], c3);
+    ct_bf(x[6], x[7], mul_i(c3));
+}
+
+// forward pass p of R stages on the thread's register set of that pass
+template <int LOGM, int R, class C>
+__device__ __forceinline__ void fwd_fft_pass(C (&x)[8], int p, uint32_t tid, const C* tab) {
+    using Tb = FftTab<LOGM>;
+    using Re = real_of<C>;
     constexpr uint32_t M = 1u << LOGM;
-    const uint32_t h = M / (2 * m);
+    if (p == 0) {  // stages 0-2: the constants do not depend on the thread
+        C c0, c1, c2, c3;
+        c0.x = Re(kSqrtHalf), c0.y = Re(kSqrtHalf);                            // exp(i pi / 4)
+        c1.x = Re(0.92387953251128675613), c1.y = Re(0.38268343236508977173);  // exp(i pi / 8)
+        c2.x = Re(0.98078528040323044913), c2.y = Re(0.19509032201612826785);  // exp(i pi / 16)
+        c3.x = Re(0.55557023301960222474), c3.y = Re(0.83146961230254523708);  // exp(5 i pi / 16)
+        fwd_stages3(x, c0, c1, c2, c3);
+        return;
+    }
+    const C* tb = tab + Tb::fwd_off(p);
     if (R == 3) {
-        const uint32_t q = h / 4, j0 = tid % q;
-        if (COMPACT && q == 1) {  // h = 4: stage 1 twiddles 1, w8, i, w8^3; stage 2 1, i; stage 3 1
-            {
-                const C t = csubd(x[0], x[4]);
-                x[0] = cadd(x[0], x[4]);
-                x[4] = t;
-            }
-            dif_bf(x[1], x[5], tb[1]);
-            {
-                const C t = mul_i(csubd(x[2], x[6]));
-                x[2] = cadd(x[2], x[6]);
-                x[6] = t;
-            }
-            dif_bf(x[3], x[7], tb[3]);
-            // stage 2: twiddle 1 on the slot pairs (0,2), (4,6) and i on (1,3), (5,7)
-#pragma unroll
-            for (int g = 0; g < 8; g += 4) {
-                C t = csubd(x[g], x[g + 2]);
-                x[g] = cadd(x[g], x[g + 2]);
-                x[g + 2] = t;
-                t = mul_i(csubd(x[g + 1], x[g + 3]));
-                x[g + 1] = cadd(x[g + 1], x[g + 3]);
-                x[g + 3] = t;
-            }
-#pragma unroll
-            for (int r = 0; r < 8; r += 2) {
-                const C t = csubd(x[r], x[r + 1]);
-                x[r] = cadd(x[r], x[r + 1]);
-                x[r + 1] = t;
-            }
-            return;
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) dif_bf(x[r], x[r + 4], COMPACT ? tb[r * q + j0] : tb[(j0 + r * q) * m]);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const C w = COMPACT ? tb[4 * q + r * q + j0] : tb[(j0 + r * q) * 2 * m];
-            dif_bf(x[r], x[r + 2], w);
-            dif_bf(x[r + 4], x[r + 6], w);
-        }
-        if (COMPACT && q == 2) {  // h = 8: the last stage's twiddle is i^j0
-#pragma unroll
-            for (int r = 0; r < 8; r += 2) {
-                const C t = csubd(x[r], x[r + 1]);
-                x[r] = cadd(x[r], x[r + 1]);
-                x[r + 1] = j0 ? mul_i(t) : t;
-            }
-        } else {
-            const C w = COMPACT ? tb[6 * q + j0] : tb[j0 * 4 * m];
-#pragma unroll
-            for (int r = 0; r < 8; r += 2) dif_bf(x[r], x[r + 1], w);
-        }
+        const uint32_t m = 1u << (3 * p), k = tid / (M / (8 * m));
+        fwd_stages3(x, tb[k], tb[m + k], tb[2 * m + k], tb[3 * m + k]);
     } else if (R == 2) {
-        const uint32_t q = h / 2;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const uint32_t j0 = (2 * tid + hh) % q;
-            C* v = x + 4 * hh;
-            if (COMPACT && q == 1) {  // twiddles 1, i, 1
-                C t = csubd(v[0], v[2]);
-                v[0] = cadd(v[0], v[2]);
-                v[2] = t;
-                t = mul_i(csubd(v[1], v[3]));
-                v[1] = cadd(v[1], v[3]);
-                v[3] = t;
-                t = csubd(v[0], v[1]);
-                v[0] = cadd(v[0], v[1]);
-                v[1] = t;
-                t = csubd(v[2], v[3]);
-                v[2] = cadd(v[2], v[3]);
-                v[3] = t;
-            } else {
-                dif_bf(v[0], v[2], COMPACT ? tb[j0] : tb[j0 * m]);
-                dif_bf(v[1], v[3], COMPACT ? tb[q + j0] : tb[(j0 + q) * m]);
-                const C w = COMPACT ? tb[2 * q + j0] : tb[j0 * 2 * m];
-                dif_bf(v[0], v[1], w);
-                dif_bf(v[2], v[3], w);
-            }
-        }
+        constexpr uint32_t T = M / 8;
+        const C c0 = tb[tid], c1 = tb[T + tid], c2 = tb[2 * T + tid];
+        ct_bf(x[0], x[2], c0);
+        ct_bf(x[1], x[3], c0);
+        ct_bf(x[4], x[6], mul_i(c0));
+        ct_bf(x[5], x[7], mul_i(c0));
+        ct_bf(x[0], x[1], c1);
+        ct_bf(x[2], x[3], mul_i(c1));
+        ct_bf(x[4], x[5], c2);
+        ct_bf(x[6], x[7], mul_i(c2));
     } else {
-#pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-            if (COMPACT && h == 1) {  // twiddle 1
-                const C t = csubd(x[2 * hh], x[2 * hh + 1]);
-                x[2 * hh] = cadd(x[2 * hh], x[2 * hh + 1]);
-                x[2 * hh + 1] = t;
-            } else {
-                const uint32_t j0 = (4 * tid + hh) % h;
-                dif_bf(x[2 * hh], x[2 * hh + 1], COMPACT ? tb[j0] : tb[j0 * m]);
-            }
-        }
+        constexpr uint32_t T = M / 8;
+        const C c0 = tb[tid], c1 = tb[T + tid];
+        ct_bf(x[0], x[1], c0);
+        ct_bf(x[2], x[3], mul_i(c0));
+        ct_bf(x[4], x[5], c1);
+        ct_bf(x[6], x[7], mul_i(c1));
     }
 }
 
-template <int LOGM, int R, bool COMPACT, class C>
-__device__ __forceinline__ void dit_pass(C (&x)[8], uint32_t m, uint32_t tid, const C* tb) {
+// inverse pass p of R stages on the thread's register set of that pass
+template <int LOGM, int R, class C>
+__device__ __forceinline__ void inv_fft_pass(C (&x)[8], int p, uint32_t tid, const C* tab) {
+    using Tb = FftTab<LOGM>;
     constexpr uint32_t M = 1u << LOGM;
-    const uint32_t h = M / (2 * m);
     if (R == 3) {
-        const uint32_t q = h / 4, j0 = tid % q;
-        if (COMPACT && q == 1) {
+        const uint32_t q = M >> (3 * p + 3), j0 = tid % q;
+        const C* tb = tab + Tb::inv_off(p);
+        // half-size q: twiddle tw(4 j0 m)
+        if (q == 1) {
+#pragma unroll
+            for (int r = 0; r < 8; r += 2) dit_bf_one(x[r], x[r + 1]);
+        } else if (q == 2) {  // the twiddle is i^j0
 #pragma unroll
             for (int r = 0; r < 8; r += 2) {
-                const C t = x[r + 1];
-                x[r + 1] = csubd(x[r], t);
-                x[r] = cadd(x[r], t);
-            }
-#pragma unroll
-            for (int g = 0; g < 8; g += 4) {  // twiddle 1 on (0,2), (4,6); i (conjugated) on (1,3), (5,7)
-                C t = x[g + 2];
-                x[g + 2] = csubd(x[g], t);
-                x[g] = cadd(x[g], t);
-                t = mul_negi(x[g + 3]);
-                x[g + 3] = csubd(x[g + 1], t);
-                x[g + 1] = cadd(x[g + 1], t);
-            }
-            {
-                const C t = x[4];
-                x[4] = csubd(x[0], t);
-                x[0] = cadd(x[0], t);
-            }
-            dit_bf(x[1], x[5], tb[1]);
-            {
-                const C t = mul_negi(x[6]);
-                x[6] = csubd(x[2], t);
-                x[2] = cadd(x[2], t);
-            }
-            dit_bf(x[3], x[7], tb[3]);
-            return;
-        }
-        if (COMPACT && q == 2) {
-#pragma unroll
-            for (int r = 0; r < 8; r += 2) {
-                const C t = j0 ? mul_negi(x[r + 1]) : x[r + 1];
-                x[r + 1] = csubd(x[r], t);
-                x[r] = cadd(x[r], t);
+                C t = j0 ? mul_negi(x[r + 1]) : x[r + 1];
+                dit_bf_one(x[r], t);
+                x[r + 1] = t;
             }
         } else {
-            const C w = COMPACT ? tb[6 * q + j0] : tb[j0 * 4 * m];
+            const C w = tb[3 * q + j0];
 #pragma unroll
             for (int r = 0; r < 8; r += 2) dit_bf(x[r], x[r + 1], w);
         }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const C w = COMPACT ? tb[4 * q + r * q + j0] : tb[(j0 + r * q) * 2 * m];
-            dit_bf(x[r], x[r + 2], w);
-            dit_bf(x[r + 4], x[r + 6], w);
+        // half-size 2q: tw(2 j0 m) and i times it
+        if (q == 1) {
+            dit_bf_one(x[0], x[2]);
+            dit_bf_one(x[4], x[6]);
+            dit_bf_i(x[1], x[3]);
+            dit_bf_i(x[5], x[7]);
+        } else {
+            const C w = tb[2 * q + j0];
+            dit_bf(x[0], x[2], w);
+            dit_bf(x[4], x[6], w);
+            dit_bf(x[1], x[3], mul_i(w));
+            dit_bf(x[5], x[7], mul_i(w));
         }
+        // half-size 4q: tw(j0 m), tw((j0 + q) m) and i times them
+        if (q == 1) {
+            C w;
+            w.x = w.y = static_cast<real_of<C>>(kSqrtHalf);
+            dit_bf_one(x[0], x[4]);
+            dit_bf(x[1], x[5], w);
+            dit_bf_i(x[2], x[6]);
+            dit_bf(x[3], x[7], mul_i(w));
+        } else {
+            const C w0 = tb[j0], w1 = tb[q + j0];
+            dit_bf(x[0], x[4], w0);
+            dit_bf(x[1], x[5], w1);
+            dit_bf(x[2], x[6], mul_i(w0));
+            dit_bf(x[3], x[7], mul_i(w1));
+        }
+    } else if (R == 2) {  // tail: twiddles 1, then 1 and i
 #pragma unroll
-        for (int r = 0; r < 4; ++r) dit_bf(x[r], x[r + 4], COMPACT ? tb[r * q + j0] : tb[(j0 + r * q) * m]);
-    } else if (R == 2) {
-        const uint32_t q = h / 2;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const uint32_t j0 = (2 * tid + hh) % q;
-            C* v = x + 4 * hh;
-            if (COMPACT && q == 1) {
-                C t = v[1];
-                v[1] = csubd(v[0], t);
-                v[0] = cadd(v[0], t);
-                t = v[3];
-                v[3] = csubd(v[2], t);
-                v[2] = cadd(v[2], t);
-                t = v[2];
-                v[2] = csubd(v[0], t);
-                v[0] = cadd(v[0], t);
-                t = mul_negi(v[3]);
-                v[3] = csubd(v[1], t);
-                v[1] = cadd(v[1], t);
-            } else {
-                const C w = COMPACT ? tb[2 * q + j0] : tb[j0 * 2 * m];
-                dit_bf(v[0], v[1], w);
-                dit_bf(v[2], v[3], w);
-                dit_bf(v[0], v[2], COMPACT ? tb[j0] : tb[j0 * m]);
-                dit_bf(v[1], v[3], COMPACT ? tb[q + j0] : tb[(j0 + q) * m]);
-            }
+        for (int g = 0; g < 8; g += 4) {
+            dit_bf_one(x[g], x[g + 1]);
+            dit_bf_one(x[g + 2], x[g + 3]);
+            dit_bf_one(x[g], x[g + 2]);
+            dit_bf_i(x[g + 1], x[g + 3]);
         }
     } else {
 #pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-            if (COMPACT && h == 1) {
-                const C t = x[2 * hh + 1];
-                x[2 * hh + 1] = csubd(x[2 * hh], t);
-                x[2 * hh] = cadd(x[2 * hh], t);
-            } else {
-                const uint32_t j0 = (4 * tid + hh) % h;
-                dit_bf(x[2 * hh], x[2 * hh + 1], COMPACT ? tb[j0] : tb[j0 * m]);
-            }
-        }
+        for (int r = 0; r < 8; r += 2) dit_bf_one(x[r], x[r + 1]);
     }
 }
 
@@ -321,19 +307,18 @@ constexpr bool inv_exchange_in_warp(int p) {
     return ((1u << LOGM) >> (3 * p)) / 8 <= 32;
 }
 
-// Forward FFT of one folded, twisted polynomial by M/8 threads.  tab: the FftTab layout (in
-// shared memory); load(j, e) returns z_e for register slot j (e < M); on return x[j] holds
+// Forward FFT of one folded polynomial by M/8 threads.  tab: the FftTab layout (in shared
+// memory); load(j, e) returns z_e = a_e + i a_(e+M) for register slot j (e < M); on return x[j] holds
 // spectrum slot 8*tid + j.  sm: M elements of shared memory, which the caller must not let
 // other threads of the group still be reading when this is entered; bar() synchronises the
 // M/8 threads of the transform.
 template <int LOGM, class Load, class Bar, class C>
 __device__ __forceinline__ void fft_forward_to_regs(C* sm, uint32_t tid, const C* tab, Load load, C (&x)[8], Bar bar) {
     using Pl = NttPlan<LOGM>;
-    using Tb = FftTab<LOGM>;
     static_assert(Pl::P >= 2, "fft needs M >= 64");
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(j, pass_index<LOGM, 3>(1u, tid, j));
-    dif_pass<LOGM, 3, false>(x, 1u, tid, tab);
+    fwd_fft_pass<LOGM, 3>(x, 0, tid, tab);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
 #pragma unroll
@@ -344,11 +329,11 @@ __device__ __forceinline__ void fft_forward_to_regs(C* sm, uint32_t tid, const C
         if (p < Pl::P - 1) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[cswz_of<C>(pass_index<LOGM, 3>(m, tid, j))];
-            dif_pass<LOGM, 3, true>(x, m, tid, tab + Tb::pass_off(p));
+            fwd_fft_pass<LOGM, 3>(x, p, tid, tab);
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[cswz_of<C>(pass_index<LOGM, Pl::tail_r>(m, tid, j))];
-            dif_pass<LOGM, Pl::tail_r, true>(x, m, tid, tab + Tb::pass_off(p));
+            fwd_fft_pass<LOGM, Pl::tail_r>(x, p, tid, tab);
         }
     }
 }
@@ -360,7 +345,6 @@ template <int LOGM, class Load0, class Load1, class Bar, class C>
 __device__ __forceinline__ void fft_forward2_to_regs(C* sm0, C* sm1, uint32_t tid, const C* tab, Load0 load0,
                                                      Load1 load1, C (&x0)[8], C (&x1)[8], Bar bar) {
     using Pl = NttPlan<LOGM>;
-    using Tb = FftTab<LOGM>;
     static_assert(Pl::P >= 2, "fft needs M >= 64");
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -368,8 +352,8 @@ __device__ __forceinline__ void fft_forward2_to_regs(C* sm0, C* sm1, uint32_t ti
         x0[j] = load0(j, e);
         x1[j] = load1(j, e);
     }
-    dif_pass<LOGM, 3, false>(x0, 1u, tid, tab);
-    dif_pass<LOGM, 3, false>(x1, 1u, tid, tab);
+    fwd_fft_pass<LOGM, 3>(x0, 0, tid, tab);
+    fwd_fft_pass<LOGM, 3>(x1, 0, tid, tab);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
 #pragma unroll
@@ -388,8 +372,8 @@ __device__ __forceinline__ void fft_forward2_to_regs(C* sm0, C* sm1, uint32_t ti
                 x0[j] = sm0[e];
                 x1[j] = sm1[e];
             }
-            dif_pass<LOGM, 3, true>(x0, m, tid, tab + Tb::pass_off(p));
-            dif_pass<LOGM, 3, true>(x1, m, tid, tab + Tb::pass_off(p));
+            fwd_fft_pass<LOGM, 3>(x0, p, tid, tab);
+            fwd_fft_pass<LOGM, 3>(x1, p, tid, tab);
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -397,8 +381,8 @@ __device__ __forceinline__ void fft_forward2_to_regs(C* sm0, C* sm1, uint32_t ti
                 x0[j] = sm0[e];
                 x1[j] = sm1[e];
             }
-            dif_pass<LOGM, Pl::tail_r, true>(x0, m, tid, tab + Tb::pass_off(p));
-            dif_pass<LOGM, Pl::tail_r, true>(x1, m, tid, tab + Tb::pass_off(p));
+            fwd_fft_pass<LOGM, Pl::tail_r>(x0, p, tid, tab);
+            fwd_fft_pass<LOGM, Pl::tail_r>(x1, p, tid, tab);
         }
     }
 }
@@ -412,9 +396,8 @@ template <int LOGM, class Store, class Bar, class C>
 __device__ __forceinline__ void fft_inverse_from_regs(C* sm, uint32_t tid, const C* tab, C (&x)[8], Store store,
                                                       Bar bar) {
     using Pl = NttPlan<LOGM>;
-    using Tb = FftTab<LOGM>;
     constexpr uint32_t mt = 1u << (3 * (Pl::P - 1));
-    dit_pass<LOGM, Pl::tail_r, true>(x, mt, tid, tab + Tb::pass_off(Pl::P - 1));
+    inv_fft_pass<LOGM, Pl::tail_r>(x, Pl::P - 1, tid, tab);
 #pragma unroll
     for (int j = 0; j < 8; ++j) sm[cswz_of<C>(pass_index<LOGM, Pl::tail_r>(mt, tid, j))] = x[j];
     if (inv_exchange_in_warp<LOGM>(Pl::P - 2)) __syncwarp();
@@ -424,8 +407,7 @@ __device__ __forceinline__ void fft_inverse_from_regs(C* sm, uint32_t tid, const
         const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[cswz_of<C>(pass_index<LOGM, 3>(m, tid, j))];
-        if (p == 0) dit_pass<LOGM, 3, false>(x, m, tid, tab);
-        else dit_pass<LOGM, 3, true>(x, m, tid, tab + Tb::pass_off(p));
+        inv_fft_pass<LOGM, 3>(x, p, tid, tab);
         if (p > 0) {
             // each pass reads and writes its own per-thread set and the sets partition [0, M), so
             // the write needs no barrier; the read of pass p - 1 does

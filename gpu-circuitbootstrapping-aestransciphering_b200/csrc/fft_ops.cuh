@@ -72,10 +72,6 @@ __device__ __forceinline__ int64_t prepared_offset(uint64_t x, uint64_t Q, uint6
     return static_cast<int64_t>(t >> ign);
 }
 
-__device__ __forceinline__ uint32_t pack_digits(int32_t re, int32_t im) {
-    return (static_cast<uint32_t>(re) & 0xffffu) | (static_cast<uint32_t>(im) << 16);
-}
-
 // zeta^e from the half table: register slot j of the first/last pass holds e = tid + j*M/8,
 // so e < M/2 exactly for j < 4; above, zeta^e = i * conj(zeta^(M-e)) = swapped components.
 template <int LOGM>
@@ -126,30 +122,32 @@ __device__ __forceinline__ double centred_double(uint64_t x, uint64_t Q, uint64_
                                           : static_cast<int64_t>(x));
 }
 
-// The biased digit fields (digit + 2^(gbits-1)) of one folded pair (a_e, a_(e+M)): packed in
-// one 32-bit word for digits of up to 15 bits (re in the low half-word), two words for wider
-// digits (the 2 x 18-bit gadget).
-template <bool WIDE>
-struct DigitPair {
-    using T = uint32_t;
-    __device__ static __forceinline__ T pack(uint32_t re, uint32_t im) { return re | (im << 16); }
-    __device__ static __forceinline__ double2 unpack(T v, int32_t bias) {
-        return make_double2(static_cast<double>(static_cast<int32_t>(v & 0xffffu) - bias),
-                            static_cast<double>(static_cast<int32_t>(v >> 16) - bias));
+// An unsigned field below 2^32 minus an integer bias, in FP64 / FP32 (exact): the field is the
+// low mantissa word of 2^52 + field (2^23 + field, fields below 2^23), so one subtraction of
+// 2^52 + bias replaces an integer conversion, which runs at a quarter of the FP64 rate.
+struct DigitBias {
+    double d;
+    __device__ __forceinline__ explicit DigitBias(uint32_t bias) : d(0x1p52 + bias) {}
+    __device__ __forceinline__ double operator()(uint32_t field) const {
+        return __hiloint2double(0x43300000, static_cast<int>(field)) - d;
     }
 };
-template <>
-struct DigitPair<true> {
-    using T = uint2;
-    __device__ static __forceinline__ T pack(uint32_t re, uint32_t im) { return make_uint2(re, im); }
-    __device__ static __forceinline__ double2 unpack(T v, int32_t bias) {
-        return make_double2(static_cast<double>(static_cast<int32_t>(v.x) - bias),
-                            static_cast<double>(static_cast<int32_t>(v.y) - bias));
-    }
+struct DigitBiasF {
+    float f;
+    __device__ __forceinline__ explicit DigitBiasF(uint32_t bias) : f(8388608.0f + static_cast<float>(bias)) {}
+    __device__ __forceinline__ float operator()(uint32_t field) const { return __uint_as_float(0x4b000000u | field) - f; }
 };
 
-// gadget digits wider than the packed 16-bit fields take the two-word form
-__host__ __device__ constexpr bool wide_digits(int gbits) { return gbits > 15; }
+// Digit pair (re, im) of the folded pair at position e of an accumulator in offset form
+// (k_blind_rotate_fft): bits [shift, shift + gbits) of both words, less the digit bias.  The
+// words are read where the transform loads them; a thread's positions are its own, so the
+// digits need no buffer and no barrier.
+template <uint32_t M>
+__device__ __forceinline__ double2 offset_digit_pair(const int64_t* acc, uint32_t e, int shift, uint32_t fmask,
+                                                     const DigitBias& bias) {
+    return make_double2(bias(static_cast<uint32_t>(static_cast<uint64_t>(acc[e]) >> shift) & fmask),
+                        bias(static_cast<uint32_t>(static_cast<uint64_t>(acc[e + M]) >> shift) & fmask));
+}
 
 template <int LOGN>
 struct BrFftCfg {

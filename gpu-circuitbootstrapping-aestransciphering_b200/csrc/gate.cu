@@ -113,7 +113,6 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS) k
     double2* fs = reinterpret_cast<double2*>(smem);                 // [2][M]
     double2* tab = fs + 2 * M;                                      // FftTab<LOGM>
     TT* acc = reinterpret_cast<TT*>(tab + Tb::size());             // [2][N] torus values
-    uint32_t* dig = reinterpret_cast<uint32_t*>(acc + 2 * N);      // [2][levels][M] packed pairs
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -123,6 +122,8 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS) k
     constexpr uint32_t W = 8 * sizeof(TT);  // torus width: 32 or 64 bits
     TT off = TT(1) << (W - levels * bg - 1);  // rounding of the dropped bits
     for (uint32_t k = 0; k < levels; ++k) off += (TT(1) << (bg - 1)) << (W - (k + 1) * bg);
+    const uint32_t fmask = (1u << bg) - 1u;
+    const DigitBias bias(1u << (bg - 1));
     auto half_bar = [h]() {
         if (h == 0) asm volatile("bar.sync 1, %0;" ::"n"(TH) : "memory");
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
@@ -162,31 +163,18 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS) k
         for (uint32_t step = 0; step < a.n; ++step) {
             const uint32_t at = ms(a.reqs ? __ldg(a1 + step) : gate_a(a.gate, __ldg(a1 + step), __ldg(a2 + step)));
             if (at == 0) continue;  // X^0 - 1 = 0: the step adds nothing (uniform over the CTA)
-            for (uint32_t e = ht; e < M; e += TH) {
-                const TT wr = my_acc[e] + off, wi = my_acc[e + M] + off;
-                uint32_t* dst = dig + h * levels * M + e;
-                for (uint32_t k = 0; k < levels; ++k) {
-                    const uint32_t s = W - (k + 1) * bg, mask = (1u << bg) - 1, half = 1u << (bg - 1);
-                    const int32_t dr = static_cast<int32_t>((wr >> s) & mask) - static_cast<int32_t>(half);
-                    const int32_t di = static_cast<int32_t>((wi >> s) & mask) - static_cast<int32_t>(half);
-                    dst[k * M] = (static_cast<uint32_t>(dr) & 0xffffu) | (static_cast<uint32_t>(di) << 16);
-                }
-            }
-            half_bar();
             const double2* ek = a.bskf + static_cast<size_t>(step) * l2 * 2 * M + ht;
             double2 y0[8], y1[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) y0[j] = y1[j] = make_double2(0.0, 0.0);
             for (uint32_t d = 0; d < levels; ++d) {
-                const uint32_t* dsrc = dig + (h * levels + d) * M;
+                const uint32_t sft = W - (d + 1) * bg;
                 double2 x[8];
                 fft_forward_to_regs<LOGM>(
                     my_fs, ht, tab,
-                    [&](int j, uint32_t e) {
-                        const uint32_t v = dsrc[e];
-                        const double re = static_cast<double>(static_cast<int16_t>(v & 0xffffu));
-                        const double im = static_cast<double>(static_cast<int16_t>(v >> 16));
-                        return cmul(make_double2(re, im), gate_twist<LOGM>(tws, j, e));
+                    [&](int, uint32_t e) {
+                        return make_double2(bias(static_cast<uint32_t>((my_acc[e] + off) >> sft) & fmask),
+                                            bias(static_cast<uint32_t>((my_acc[e + M] + off) >> sft) & fmask));
                     },
                     x, half_bar);
                 const double2* k0 = ek + static_cast<size_t>(2 * d + h) * 2 * M;
@@ -232,6 +220,7 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS) k
                 const TT v = (s < N) ? tsm[s] : TT(0) - tsm[s - N];
                 my_acc[i] += v - tsm[i];
             }
+            half_bar();  // tsm is the next step's exchange buffer
         }
         __syncthreads();
         // sample extract of coefficient 0: a'_0 = a_0, a'_i = -a_(N-i), b' = b_0
@@ -291,7 +280,6 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS)
     float2* fs = reinterpret_cast<float2*>(smem);                   // [2][LIMBS][M]
     float2* tab = fs + 2 * LIMBS * M;                               // FftTab<LOGM> in FP32
     uint32_t* acc = reinterpret_cast<uint32_t*>(tab + Tb::size());  // [2][N] torus values
-    uint32_t* dig = acc + 2 * N;                                    // [2][levels][M] packed pairs
     const float2* tws = tab + Tb::twist_off();
     const uint32_t tid = threadIdx.x, h = tid / TH, ht = tid % TH;
     uint32_t* my_acc = acc + h * N;
@@ -299,6 +287,8 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS)
     const uint32_t levels = a.levels, bg = a.bg_bits, l2 = 2 * levels;
     uint32_t off = 1u << (32 - levels * bg - 1);  // rounding of the dropped bits
     for (uint32_t k = 0; k < levels; ++k) off += (1u << (bg - 1)) << (32 - (k + 1) * bg);
+    const uint32_t fmask = (1u << bg) - 1u;
+    const DigitBiasF bias(1u << (bg - 1));
     auto half_bar = [h]() {
         if (h == 0) asm volatile("bar.sync 1, %0;" ::"n"(TH) : "memory");
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
@@ -327,17 +317,6 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS)
         for (uint32_t step = 0; step < a.n; ++step) {
             const uint32_t at = ms(a.reqs ? __ldg(a1 + step) : gate_a(a.gate, __ldg(a1 + step), __ldg(a2 + step)));
             if (at == 0) continue;  // X^0 - 1 = 0: the step adds nothing (uniform over the CTA)
-            for (uint32_t e = ht; e < M; e += TH) {
-                const uint32_t wr = my_acc[e] + off, wi = my_acc[e + M] + off;
-                uint32_t* dst = dig + h * levels * M + e;
-                for (uint32_t k = 0; k < levels; ++k) {
-                    const uint32_t s = 32 - (k + 1) * bg, mask = (1u << bg) - 1, half = 1u << (bg - 1);
-                    const int32_t dr = static_cast<int32_t>((wr >> s) & mask) - static_cast<int32_t>(half);
-                    const int32_t di = static_cast<int32_t>((wi >> s) & mask) - static_cast<int32_t>(half);
-                    dst[k * M] = (static_cast<uint32_t>(dr) & 0xffffu) | (static_cast<uint32_t>(di) << 16);
-                }
-            }
-            half_bar();
             const float2* ek = a.bskf32 + static_cast<size_t>(step) * l2 * 2 * LIMBS * M + ht;
             float2 y[2][LIMBS][8];
 #pragma unroll
@@ -347,15 +326,13 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) y[c][l][j] = make_float2(0.f, 0.f);
             for (uint32_t d = 0; d < levels; ++d) {
-                const uint32_t* dsrc = dig + (h * levels + d) * M;
+                const uint32_t sft = 32 - (d + 1) * bg;
                 float2 x[8];
                 fft_forward_to_regs<LOGM>(
                     my_fs, ht, tab,
-                    [&](int j, uint32_t e) {
-                        const uint32_t v = dsrc[e];
-                        const float re = static_cast<float>(static_cast<int16_t>(v & 0xffffu));
-                        const float im = static_cast<float>(static_cast<int16_t>(v >> 16));
-                        return cmul(make_float2(re, im), gate_twist<LOGM>(tws, j, e));
+                    [&](int, uint32_t e) {
+                        return make_float2(bias(((my_acc[e] + off) >> sft) & fmask),
+                                           bias(((my_acc[e + M] + off) >> sft) & fmask));
                     },
                     x, half_bar);
                 const float2* kr = ek + static_cast<size_t>(2 * d + h) * 2 * LIMBS * M;  // [column][limb][M]
@@ -418,6 +395,7 @@ __global__ void __launch_bounds__(GateCfg<LOGN>::T, GateCfg<LOGN>::MIN_BLOCKS)
                 const uint32_t v = (s < N) ? tsm[s] : 0u - tsm[s - N];
                 my_acc[i] += v - tsm[i];
             }
+            half_bar();  // tsm is the next step's exchange buffer
         }
         __syncthreads();
         // sample extract of coefficient 0: a'_0 = a_0, a'_i = -a_(N-i), b' = b_0
@@ -458,8 +436,7 @@ __global__ void __launch_bounds__(GateMbCfg<LOGN>::T, GateMbCfg<LOGN>::MIN_BLOCK
     double2* fs = reinterpret_cast<double2*>(smem);             // [2][M]
     double2* tab = fs + 2 * M;                                  // FftTab<LOGM>
     TT* acc = reinterpret_cast<TT*>(tab + Tb::size());         // [2][N] torus values
-    uint32_t* dig = reinterpret_cast<uint32_t*>(acc + 2 * N);  // [2][levels][M] packed pairs
-    double2* cbuf = reinterpret_cast<double2*>(dig + 2 * a.levels * M);  // [MB][8][T]
+    double2* cbuf = reinterpret_cast<double2*>(acc + 2 * N);    // [MB][8][T]
     const double2* tws = tab + Tb::twist_off();
     const uint32_t ct = blockIdx.x, tid = threadIdx.x;
     const uint32_t h = tid / TH, ht = tid % TH;
@@ -469,6 +446,8 @@ __global__ void __launch_bounds__(GateMbCfg<LOGN>::T, GateMbCfg<LOGN>::MIN_BLOCK
     constexpr uint32_t W = 8 * sizeof(TT);
     TT off = TT(1) << (W - levels * bg - 1);
     for (uint32_t k = 0; k < levels; ++k) off += (TT(1) << (bg - 1)) << (W - (k + 1) * bg);
+    const uint32_t fmask = (1u << bg) - 1u;
+    const DigitBias bias(1u << (bg - 1));
     auto half_bar = [h]() {
         if (h == 0) asm volatile("bar.sync 1, %0;" ::"n"(TH) : "memory");
         else asm volatile("bar.sync 2, %0;" ::"n"(TH) : "memory");
@@ -525,37 +504,22 @@ __global__ void __launch_bounds__(GateMbCfg<LOGN>::T, GateMbCfg<LOGN>::MIN_BLOCK
                 for (int j = 0; j < 8; ++j) {
                     const uint32_t r3 = ((j & 1) << 2) | (j & 2) | ((j >> 2) & 1);
                     const uint32_t k = (at[i] * r3) & 7u;
-                    double2 w = tab[(k & 3u) * (M / 8)];
-                    if (k & 4u) w = make_double2(-w.x, -w.y);
-                    const double2 v = cmul(ub, w);
+                    const double2 v = cmul(ub, omega8<double2>(k));
                     cbuf[(i * 8 + j) * T + tid] = make_double2(v.x - 1.0, v.y);
                 }
             }
-            for (uint32_t e = ht; e < M; e += TH) {
-                const TT wr = my_acc[e] + off, wi = my_acc[e + M] + off;
-                uint32_t* dst = dig + h * levels * M + e;
-                for (uint32_t k = 0; k < levels; ++k) {
-                    const uint32_t sft = W - (k + 1) * bg, mask = (1u << bg) - 1, half = 1u << (bg - 1);
-                    const int32_t dr = static_cast<int32_t>((wr >> sft) & mask) - static_cast<int32_t>(half);
-                    const int32_t di = static_cast<int32_t>((wi >> sft) & mask) - static_cast<int32_t>(half);
-                    dst[k * M] = (static_cast<uint32_t>(dr) & 0xffffu) | (static_cast<uint32_t>(di) << 16);
-                }
-            }
-            half_bar();
             const double2* gk = a.bskf + static_cast<size_t>(g) * KS * kstride + ht;
             double2 y0[8], y1[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) y0[j] = y1[j] = make_double2(0.0, 0.0);
             for (uint32_t d = 0; d < levels; ++d) {
-                const uint32_t* dsrc = dig + (h * levels + d) * M;
+                const uint32_t sft = W - (d + 1) * bg;
                 double2 x[8];
                 fft_forward_to_regs<LOGM>(
                     my_fs, ht, tab,
-                    [&](int j, uint32_t e) {
-                        const uint32_t v = dsrc[e];
-                        const double re = static_cast<double>(static_cast<int16_t>(v & 0xffffu));
-                        const double im = static_cast<double>(static_cast<int16_t>(v >> 16));
-                        return cmul(make_double2(re, im), gate_twist<LOGM>(tws, j, e));
+                    [&](int, uint32_t e) {
+                        return make_double2(bias(static_cast<uint32_t>((my_acc[e] + off) >> sft) & fmask),
+                                            bias(static_cast<uint32_t>((my_acc[e + M] + off) >> sft) & fmask));
                     },
                     x, half_bar);
                 const double2* k0 = gk + static_cast<size_t>(2 * d + h) * 2 * M;
@@ -670,8 +634,7 @@ __global__ void __launch_bounds__(256) k_gate_keyswitch(const uint32_t* __restri
 template <int LOGN, typename TT>
 static cudaError_t gate_br_launch(const GateArgs& a, uint32_t grid, cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
-    const size_t smem = (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) + 2ull * N * sizeof(TT) +
-                        2ull * a.levels * M * sizeof(uint32_t);
+    const size_t smem = (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) + 2ull * N * sizeof(TT);
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -689,7 +652,7 @@ template <int LOGN, typename TT, int MB>
 static cudaError_t gate_br_mb_launch(const GateArgs& a, uint32_t grid, cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
     const size_t smem = (2ull * M + FftTab<LOGN - 1>::size()) * sizeof(double2) + 2ull * N * sizeof(TT) +
-                        2ull * a.levels * M * sizeof(uint32_t) + MB * 8ull * GateMbCfg<LOGN>::T * sizeof(double2);
+                        MB * 8ull * GateMbCfg<LOGN>::T * sizeof(double2);
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -706,8 +669,7 @@ static cudaError_t gate_br_mb_launch(const GateArgs& a, uint32_t grid, cudaStrea
 template <int LOGN, int LIMBS>
 static cudaError_t gate_br_f32_launch(const GateArgs& a, uint32_t grid, cudaStream_t s) {
     constexpr uint32_t N = 1u << LOGN, M = N / 2;
-    const size_t smem = (2ull * LIMBS * M + FftTab<LOGN - 1>::size()) * sizeof(float2) + 2ull * N * sizeof(uint32_t) +
-                        2ull * a.levels * M * sizeof(uint32_t);
+    const size_t smem = (2ull * LIMBS * M + FftTab<LOGN - 1>::size()) * sizeof(float2) + 2ull * N * sizeof(uint32_t);
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
