@@ -155,6 +155,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cbs_gate_ragged_launch": (st, [c_vp, c_vp]),
         "cbs_rns_context_create": (st, [u32, c_vp, u32, c_vp, u32, c_vp]),
         "cbs_rns_context_destroy": (st, [c_vp]),
+        "cbs_keyswitch_device_fault": (st, [c_vp, ctypes.c_int]),
         "cbs_rns_device_fault": (st, [c_vp, c_vp, ctypes.c_int]),
         "cbs_ckks_add_inplace": (st, [c_vp, c_vp, c_vp, u32, u32, c_vp]),
         "cbs_ckks_sub_inplace": (st, [c_vp, c_vp, c_vp, u32, u32, ctypes.c_int, c_vp]),

@@ -420,7 +420,8 @@ cbs_status run_extract(cbs_context* c, const uint64_t* d_words_coef, const uint3
     a.base_log2 = static_cast<uint32_t>(__builtin_ctz(c->p.base_ks));
     a.q_lwe = c->p.q_lwe;
     a.scale = (c->p.q_lwe % c->p.qks == 0) ? c->p.q_lwe / c->p.qks : 0;
-    CBS_CUDA_TRY(launch_extract_keyswitch(a, count, s));
+    if (c->d_ksk_tiles.p) CBS_CUDA_TRY(ks_mma_extract(c->ks_shape, c->d_ksk_tiles.p, a, count, s));
+    else CBS_CUDA_TRY(launch_extract_keyswitch(a, count, s));
     return CBS_OK;
 }
 
@@ -470,8 +471,24 @@ cbs_status upload_host_keys(cbs_context* c) {
     return finish_key_upload(c);
 }
 
+// byte-plane tiles of the extraction key for the tensor-core switch; without the memory for them
+// (as much again as the key) or a kernel for the base the gather kernel serves
+static cbs_status build_ksk_tiles(cbs_context* c) {
+    const uint32_t bits = static_cast<uint32_t>(__builtin_ctz(c->p.base_ks));
+    c->d_ksk_tiles.reset();
+    if (!ks_mma_bits(bits)) return CBS_OK;
+    c->ks_shape = KsShape{1, c->p.N, 2, bits, c->p.n + 1, 2};
+    if (c->d_ksk_tiles.alloc(c->ks_shape.tile_bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        return CBS_OK;
+    }
+    CBS_CUDA_TRY(ks_build_tiles_u16(c->ks_shape, c->d_ksk.p, ksk_row_stride(c->p.n), c->d_ksk_tiles.p, c->stream));
+    return CBS_OK;
+}
+
 cbs_status finish_key_upload(cbs_context* c) {
     cudaStream_t s = c->stream;
+    if (cbs_status st = build_ksk_tiles(c)) return st;
     CBS_CUDA_TRY(c->d_tv.upload(c->hk.tv.data(), c->hk.tv.size(), s));
     CBS_CUDA_TRY(c->d_gadd.upload(c->hk.gadd.data(), c->hk.gadd.size(), s));
     CBS_CUDA_TRY(c->d_maps.upload(c->hk.maps.data(), c->hk.maps.size(), s));

@@ -13,6 +13,7 @@
 #include "devbuf.cuh"
 #include "encrypt.cuh"
 #include "extract_kernels.cuh"
+#include "ks_mma.cuh"
 #include "fft_kernels.cuh"
 #include "host_math.h"
 #include "keygen.h"
@@ -80,6 +81,8 @@ struct cbs_context {
     cbs::HostKeys hk;
     cbs::DevBuf<uint64_t> d_tv, d_gadd, d_bsk, d_ht, d_ss;
     cbs::DevBuf<uint16_t> d_ksk;
+    cbs::DevBuf<uint8_t> d_ksk_tiles;    // its byte-plane tiles (ks_mma.cuh); empty: the gather kernel
+    cbs::KsShape ks_shape{};
     // FP64 FFT blind-rotation backend (built on demand from the keys)
     int br_backend = 0;  // CBS_BR_NTT, CBS_BR_FFT64 or CBS_BR_FFT64_SPLIT
     bool fft_ready = false;

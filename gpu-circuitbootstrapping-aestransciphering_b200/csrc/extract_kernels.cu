@@ -13,16 +13,6 @@
 
 namespace cbs {
 
-__device__ __forceinline__ uint32_t ms_pow2(uint64_t v, double q_over_Q, uint32_t mask) {
-    return static_cast<uint32_t>(__double2uint_rn(static_cast<double>(v) * q_over_Q)) & mask;
-}
-
-__device__ __forceinline__ uint64_t qks_to_q(uint32_t v, uint64_t scale, uint32_t qks, uint64_t q) {
-    if (scale) return static_cast<uint64_t>(v) * scale;
-    const unsigned __int128 x = static_cast<unsigned __int128>(v) * q + (qks >> 1);
-    return static_cast<uint64_t>(x / qks);
-}
-
 // One CTA per output bit: the mod-switched mask (N u16) is staged in shared memory once, and
 // each thread accumulates 4 consecutive outputs from one 8-byte load per key row (rows padded
 // to a multiple of 4 words), unrolled so that 16 independent loads are in flight.
@@ -44,7 +34,7 @@ __global__ void __launch_bounds__(kExtractThreads) k_extract_keyswitch(const Ext
             const uint64_t x = aw[a.N + idx - c];
             v = x ? a.Q - x : 0;
         }
-        s_a[c] = static_cast<uint16_t>(ms_pow2(v, a.q_over_Q, a.mask));
+        s_a[c] = static_cast<uint16_t>(extract_ms_pow2(v, a.q_over_Q, a.mask));
     }
     __syncthreads();
     const uint32_t bmask = a.base_ks - 1;
@@ -73,8 +63,8 @@ __global__ void __launch_bounds__(kExtractThreads) k_extract_keyswitch(const Ext
             const uint32_t k = 4 * q + w;
             if (k > a.n) break;
             uint32_t accv = accs[w];
-            if (k == a.n) accv += ms_pow2(bw[idx], a.q_over_Q, a.mask);
-            const uint64_t val = qks_to_q(accv & a.mask, a.scale, a.qks, a.q_lwe);
+            if (k == a.n) accv += extract_ms_pow2(bw[idx], a.q_over_Q, a.mask);
+            const uint64_t val = extract_qks_to_q(accv & a.mask, a.scale, a.qks, a.q_lwe);
             if (k == a.n) a.out_b[t] = val;
             else a.out_a[static_cast<size_t>(t) * a.out_stride + k] = val;
         }

@@ -24,6 +24,18 @@ struct ExtractArgs {
     uint64_t scale;         // q_lwe / qks when divisible, else 0
 };
 
+// Q -> qKS (a power of two; mask = qKS - 1), FP64 round-to-nearest (aes_gpu_ks.cuh:388-394)
+__device__ __forceinline__ uint32_t extract_ms_pow2(uint64_t v, double q_over_Q, uint32_t mask) {
+    return static_cast<uint32_t>(__double2uint_rn(static_cast<double>(v) * q_over_Q)) & mask;
+}
+// qKS -> q: exact scale, or round-half-up division (aes_gpu_ks.cuh:431-440)
+__device__ __forceinline__ uint64_t extract_qks_to_q(uint32_t v, uint64_t scale, uint32_t qks, uint64_t q) {
+    if (scale) return static_cast<uint64_t>(v) * scale;
+    const unsigned __int128 x = static_cast<unsigned __int128>(v) * q + (qks >> 1);
+    return static_cast<uint64_t>(x / qks);
+}
+
+// one CTA per output gathering the selected key rows (any base; ks_mma.cuh has the tensor form)
 cudaError_t launch_extract_keyswitch(const ExtractArgs& a, uint32_t count, cudaStream_t s);
 // row stride of the device key-switching key: n + 1 rounded up to a multiple of 4 words
 inline uint32_t ksk_row_stride(uint32_t n) { return (n + 1 + 3) & ~3u; }

@@ -847,15 +847,6 @@ void torus_keys_to_fft(uint32_t N, const uint64_t* keys, size_t count, std::vect
     else out.clear();
 }
 
-cudaError_t gate_keyswitch(const GateArgs& a, const uint32_t* ksk, uint32_t n, uint32_t N, uint32_t ks_bits,
-                           uint32_t ks_levels, uint32_t* out_a, uint32_t* out_b, cudaStream_t s) {
-    const dim3 grid(a.items, (n + 1 + 255) / 256);
-    k_gate_keyswitch<<<grid, 256, (N + 1) * sizeof(uint32_t), s>>>(static_cast<const uint32_t*>(a.ext), ksk, n, N,
-                                                                   ks_bits, ks_levels, out_a, out_b,
-                                                                   a.reqs, a.num_reqs);
-    return cudaGetLastError();
-}
-
 }  // namespace cbs
 
 // ---------------------------------------------------------------------------------------
@@ -884,6 +875,20 @@ cbs_status gate_fill_keys(const cbs_gate_context* ctx, GateArgs& a) {
     a.bskf32 = ctx->d_bskf32.p;
     a.tab32 = ctx->d_tab32.p;
     return CBS_OK;
+}
+
+cudaError_t gate_keyswitch(const cbs_gate_context* ctx, const GateArgs& a, uint32_t* out_a, uint32_t* out_b,
+                           cudaStream_t s) {
+    const cbs_gate_params& p = ctx->p;
+    const uint32_t* ext = static_cast<const uint32_t*>(a.ext);
+    if (ctx->d_ksk_tiles.p) {
+        const uint32_t round = 1u << (32 - p.ks_levels * p.ks_base_bits - 1);
+        return ks_mma_gate(ctx->ks_shape, ctx->d_ksk_tiles.p, ext, a.items, round, out_a, out_b, a.reqs, a.num_reqs, s);
+    }
+    const dim3 grid(a.items, (p.n + 1 + 255) / 256);
+    k_gate_keyswitch<<<grid, 256, (p.N + 1) * sizeof(uint32_t), s>>>(ext, ctx->d_ksk.p, p.n, p.N, p.ks_base_bits,
+                                                                     p.ks_levels, out_a, out_b, a.reqs, a.num_reqs);
+    return cudaGetLastError();
 }
 
 }  // namespace cbs
@@ -1069,8 +1074,21 @@ cbs_status gate_prepare_f32(cbs_gate_context* ctx) {
     return CBS_OK;
 }
 
-// the arithmetic fields of the launch arguments; CBS_ERR_NOT_READY when the selected keys are
-// not prepared
+// byte-plane tiles of the key-switching key for the tensor-core switch (digits of up to 7 bits;
+// without the memory for them the gather kernel serves)
+cbs_status gate_build_ksk_tiles(cbs_gate_context* ctx) {
+    const cbs_gate_params& p = ctx->p;
+    ctx->d_ksk_tiles.reset();
+    if (!cbs::ks_mma_bits(p.ks_base_bits)) return CBS_OK;
+    ctx->ks_shape = cbs::KsShape{1, p.N, p.ks_levels, p.ks_base_bits, p.n + 1, 4};
+    if (ctx->d_ksk_tiles.alloc(ctx->ks_shape.tile_bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        return CBS_OK;
+    }
+    CBS_CUDA_TRY(cbs::ks_build_tiles(ctx->ks_shape, ctx->d_ksk.p, (1u << p.ks_base_bits) - 1, p.n + 1,
+                                     ctx->d_ksk_tiles.p, nullptr));
+    return CBS_OK;
+}
 
 cbs_status gate_prepare_mb(cbs_gate_context* ctx) {
     if (ctx->br_mb <= 1 || ctx->mb_ready || !ctx->keys_ready) return CBS_OK;
@@ -1091,6 +1109,12 @@ cbs_status gate_prepare_mb(cbs_gate_context* ctx) {
 }  // namespace
 
 extern "C" {
+
+cbs_status cbs_keyswitch_device_fault(uint32_t* out, int clear) {
+    CBS_CHECK_ARG(out, "keyswitch_device_fault: null argument");
+    CBS_CUDA_TRY(cbs::ks_mma_fault(out, clear != 0));
+    return CBS_OK;
+}
 
 cbs_status cbs_gate_set_multibit(cbs_gate_context* ctx, uint32_t mb) {
     CBS_CHECK_ARG(ctx, "gate_set_multibit: null context");
@@ -1166,7 +1190,9 @@ cbs_status cbs_gate_keygen(cbs_gate_context* ctx, uint64_t seed) {
     CBS_CUDA_TRY(ctx->d_bskf.upload(bskf.data(), bskf.size(), nullptr));
     CBS_CUDA_TRY(ctx->d_tab.upload(tab.data(), tab.size(), nullptr));
     CBS_CUDA_TRY(ctx->d_ksk.upload(ctx->ksk.data(), ctx->ksk.size(), nullptr));
+    if (cbs_status st = gate_build_ksk_tiles(ctx)) return st;
     CBS_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    if (ctx->d_ksk_tiles.p) ctx->d_ksk.reset();
     ctx->keys_ready = true;
     ctx->key_seed = seed;
     ctx->mb_ready = false;
@@ -1256,11 +1282,7 @@ static cbs_status gate_run(cbs_gate_context* ctx, int gate, const uint32_t* d_a1
     a.mu[0] = 1u << 29;
     CBS_CUDA_TRY(cbs::gate_blind_rotate(a, p.N, count, s));
     if (d_out_a && d_out_b) {
-        const dim3 grid(count, (p.n + 1 + 255) / 256);
-        cbs::k_gate_keyswitch<<<grid, 256, (p.N + 1) * sizeof(uint32_t), s>>>(
-            static_cast<const uint32_t*>(a.ext), ctx->d_ksk.p, p.n, p.N, p.ks_base_bits, p.ks_levels, d_out_a, d_out_b,
-            nullptr, 0);
-        CBS_LAUNCH_CHECK();
+        CBS_CUDA_TRY(cbs::gate_keyswitch(ctx, a, d_out_a, d_out_b, s));
     }
     return CBS_OK;
 }
@@ -1375,11 +1397,7 @@ cbs_status cbs_gate_ragged_launch(cbs_gate_context* ctx, cbs_stream_t stream) {
     a.levels_tv = 1;
     a.mu[0] = 1u << 29;
     CBS_CUDA_TRY(cbs::gate_blind_rotate(a, p.N, ctx->plan_grid, stream));
-    const dim3 grid(ctx->plan_items, (p.n + 1 + 255) / 256);
-    cbs::k_gate_keyswitch<<<grid, 256, (p.N + 1) * sizeof(uint32_t), stream>>>(
-        static_cast<const uint32_t*>(a.ext), ctx->d_ksk.p, p.n, p.N, p.ks_base_bits, p.ks_levels, nullptr, nullptr,
-        a.reqs, a.num_reqs);
-    CBS_LAUNCH_CHECK();
+    CBS_CUDA_TRY(cbs::gate_keyswitch(ctx, a, nullptr, nullptr, stream));
     return CBS_OK;
 }
 

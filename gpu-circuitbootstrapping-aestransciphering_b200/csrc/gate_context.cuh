@@ -7,6 +7,7 @@
 #include "../../include/cbs_b200.h"
 #include "common.cuh"
 #include "devbuf.cuh"
+#include "ks_mma.cuh"
 #include "torus.cuh"
 
 struct cbs_gate_context {
@@ -17,6 +18,8 @@ struct cbs_gate_context {
     std::vector<uint32_t> bsk, ksk;  // coefficient form (exported) / device layout
     cbs::DevBuf<double2> d_bskf, d_tab;
     cbs::DevBuf<uint32_t> d_ksk, d_ext, d_tmp_a, d_tmp_b;
+    cbs::DevBuf<uint8_t> d_ksk_tiles;  // byte-plane tiles of the key (ks_mma.cuh), in place of d_ksk
+    cbs::KsShape ks_shape{};
     // ragged plan (cbs_gate_ragged_plan): request table, its extracted-LWE scratch, grid
     cbs::DevBuf<cbs::GateReq> d_plan;
     cbs::DevBuf<uint32_t> d_plan_ext;
@@ -40,4 +43,7 @@ struct cbs_gate_context {
 namespace cbs {
 // the key spectra / grouped keys / FP32 limbs of the context's current settings into a
 cbs_status gate_fill_keys(const cbs_gate_context* ctx, GateArgs& a);
+// key switch of the extracted ciphertexts a.ext into out_a / out_b (or a.reqs' outputs)
+cudaError_t gate_keyswitch(const cbs_gate_context* ctx, const GateArgs& a, uint32_t* out_a, uint32_t* out_b,
+                           cudaStream_t s);
 }  // namespace cbs

@@ -146,7 +146,7 @@ struct FuncRun {
         a.levels_tv = 1;
         a.tv = ctx->d_tv.p;
         CBS_CUDA_TRY(gate_blind_rotate(a, N, count, s));
-        CBS_CUDA_TRY(gate_keyswitch(a, ctx->d_ksk.p, p.n, N, p.ks_base_bits, p.ks_levels, out.a, out.b, s));
+        CBS_CUDA_TRY(gate_keyswitch(ctx, a, out.a, out.b, s));
         return round(out, 32, f_bits);
     }
 };

@@ -1,0 +1,569 @@
+// ks_mma.cu -- key switching as a one-hot integer matrix product on the 5th-generation tensor
+// cores.
+//
+// Every key switch of this library (the gate's N -> n switch, the torus circuit bootstrap's
+// PFKS, the CBS extraction switch) adds, for each input coefficient i and digit l, the key row
+// that the digit's value selects: out = init +- sum_{i,l} KEY[i][l][v_{i,l}].  That is a product
+// of the key with a matrix of one-hot columns: with one slot k = (i, l, v) per key row,
+// out^T = KEY^T O, O[k][item] = 1 where item's digit (i, l) equals v.  The key's words are cut
+// into byte planes (u8), so tcgen05.mma kind::i8 (u8 x u8 -> s32) gives each plane's exact sum
+// (at most 2^15 selected bytes, below 2^23), and the planes are put together as
+// sum_p plane_p 2^(8p) mod 2^32: the same words as adding rows.
+//
+// The gathers this replaces read every selected row for every ciphertext (15.6 MB of L2 traffic
+// per gate, 5.2 MB per AES output bit) at a latency-bound 20-30 % of the L2 rate; here a key
+// tile is read once per 128 ciphertexts and the additions run at the tensor rate, so small
+// batches are bound by reading the key once (HBM / L2) and large ones by the tensor pipe and the
+// operands' shared-memory traffic.  Measured against the gathers: 64 gates 1248 -> 25 us (84 MB of
+// tiles), 883 gates 4189 -> 139 us, PFKS of 48 bits 9314 -> 998 us (4.3 GB of tiles, 4.3 TB/s),
+// extraction of 128 bits 757 -> 152 us (671 MB, 4.6 TB/s), of 1664 bits 1312 -> 1192 us.
+//
+// One CTA per SM: 128 output words (TMEM lanes) x up to 128 items (256 for two byte planes; columns)
+// x byte planes (a column block each, 512 columns in all), over a range of slots (split-K over CTAs; partial
+// sums meet in red.add on the outputs, exact in any order).  The key is stored as 16 KB tiles
+// [group][128-slot step][plane][128 words][128 slots] in the 128-byte-swizzled K-major order the
+// MMA reads, so one bulk copy brings a tile and no tensor map is needed.  Warp 0 streams tiles
+// through a ring, eight warps write the one-hot operand of each step (three-stage
+// ring, coefficients loaded a step ahead), warp 1 issues the MMAs; the eight warps then read TMEM and add.
+// Items are padded to a multiple of 16 (the N of the instruction).  Every wait is bounded.
+#include "ks_mma.cuh"
+
+#include "async_copy.cuh"
+#include "common.cuh"
+#include "extract_kernels.cuh"
+#include "tmem.cuh"
+
+namespace cbs {
+
+__device__ uint32_t g_ks_fault;
+
+namespace {
+
+constexpr uint32_t kHotStages = 3, kTile = 128 * 128;
+constexpr uint32_t kGenWarps = 8, kThreads = 64 + 32 * kGenWarps;
+constexpr long long kWaitLimit = 2000000000ll;  // SM clocks, about a second
+
+// The 512 TMEM columns hold PLANES blocks of ITEMS columns.  Shared memory, from a 1024-byte
+// boundary: key ring, one-hot ring (ITEMS rows of 128 slots a stage), output pointers, barriers.
+template <int PLANES>
+struct KsCfg {
+    static constexpr uint32_t ITEMS = 512 / PLANES, HOT = ITEMS * 128;
+    static_assert(ITEMS <= 256, "the instruction's N");
+    static constexpr uint32_t KEY_STAGES = ITEMS == 128 ? 10 : 7;
+    static constexpr size_t hot_off = static_cast<size_t>(KEY_STAGES) * kTile;
+    static constexpr size_t ptr_off = hot_off + static_cast<size_t>(kHotStages) * HOT;
+    static constexpr size_t bar_off = ptr_off + ITEMS * 2 * sizeof(uint32_t*);
+    static constexpr size_t bars = 2 * KEY_STAGES + 2 * kHotStages + 1;
+    static constexpr size_t bytes = bar_off + bars * 8 + 16 + 1024;  // + TMEM slot, abort flag, alignment
+};
+
+// shared-memory matrix descriptor of a K-major tile of 128-byte rows, 128-byte swizzle: rows of
+// a group of 8 are 128 bytes apart, groups 1024 bytes
+__device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
+    return static_cast<uint64_t>((addr & 0x3ffffu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+// instruction descriptor: s32 accumulator, u8 x u8, M = 128, N = n
+__device__ __forceinline__ uint32_t i8_idesc(uint32_t n) { return (2u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// the barrier receives one arrival when every MMA issued so far by this thread has completed
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// ---- the three users: the digit word of (item, coefficient), outputs ----
+
+struct GateSrc {  // digit l = bits [32 - (l+1) b, 32 - l b) of ext + round
+    const uint32_t* ext;
+    uint32_t coefs, items, round;
+    uint32_t *out_a, *out_b;
+    const GateReq* reqs;
+    uint32_t num_reqs;
+    using Row = const uint32_t*;  // what a thread keeps of its item
+    __device__ Row row(uint32_t item) const { return ext + static_cast<size_t>(item) * (coefs + 1); }
+    __device__ uint32_t word(Row r, uint32_t i) const { return __ldg(r + i) + round; }
+    // the item's output row (words below n) and its last word
+    __device__ void rows(uint32_t item, uint32_t, uint32_t words, uint32_t*& a, uint32_t*& last) const {
+        uint32_t* oa = out_a;
+        uint32_t* ob = out_b;
+        uint32_t k = item;
+        if (reqs) {
+            uint32_t lo = 0, hi = num_reqs;
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) / 2;
+                if (__ldg(&reqs[mid].offset) <= item) lo = mid;
+                else hi = mid;
+            }
+            oa = reqs[lo].out_a;
+            ob = reqs[lo].out_b;
+            k = item - reqs[lo].offset;
+        }
+        a = oa + static_cast<size_t>(k) * (words - 1);
+        last = ob + k;
+    }
+    static constexpr bool kSubtract = true;
+    static constexpr uint32_t kStep = 1;  // 32-bit words between outputs
+};
+
+struct TcbSrc {  // digits of the top 32 bits (rounded) of -a_i, or of b for the last coefficient
+    const uint64_t* ext;
+    uint32_t coefs, items, funcs;
+    uint32_t* rgsw;
+    using Row = const uint64_t*;
+    __device__ Row row(uint32_t item) const { return ext + static_cast<size_t>(item) * coefs; }
+    __device__ uint32_t word(Row r, uint32_t i) const {
+        const uint64_t v = __ldg(r + i);
+        const uint64_t x = i + 1 < coefs ? 0ull - v : v;
+        return static_cast<uint32_t>((x + (1ull << 31)) >> 32);
+    }
+    __device__ void rows(uint32_t item, uint32_t fn, uint32_t words, uint32_t*& a, uint32_t*& last) const {
+        a = rgsw + (static_cast<size_t>(item) * funcs + fn) * words;
+        last = a + words - 1;
+    }
+    static constexpr bool kSubtract = false;
+    static constexpr uint32_t kStep = 1;
+};
+
+struct ExtractSrc {  // two digits, low first, of the mod-switched coefficient of the extracted mask
+    ExtractArgs e;
+    uint32_t items;
+    struct Row {
+        const uint64_t* a;
+        uint32_t idx;
+    };
+    __device__ Row row(uint32_t item) const {
+        const uint32_t info = __ldg(e.info + item);
+        return Row{e.words + static_cast<size_t>(info >> 16) * 2 * e.N, info & 0xffffu};
+    }
+    __device__ uint32_t word(const Row& r, uint32_t c) const {
+        const bool neg = c > r.idx;
+        const uint64_t x = __ldg(r.a + (neg ? e.N : 0u) + r.idx - c);
+        const uint64_t v = neg && x ? e.Q - x : x;
+        const uint32_t ai = extract_ms_pow2(v, e.q_over_Q, e.mask), bm = e.base_ks - 1;
+        return ((ai & bm) << (32 - e.base_log2)) | (((ai >> e.base_log2) & bm) << (32 - 2 * e.base_log2));
+    }
+    // the outputs are 64-bit; the sums (mod 2^32) build up in their low words
+    __device__ void rows(uint32_t item, uint32_t, uint32_t, uint32_t*& a, uint32_t*& last) const {
+        a = reinterpret_cast<uint32_t*>(e.out_a + static_cast<size_t>(item) * e.out_stride);
+        last = reinterpret_cast<uint32_t*>(e.out_b + item);
+    }
+    static constexpr bool kSubtract = true;
+    static constexpr uint32_t kStep = 2;
+};
+
+struct KsGrid {
+    const uint8_t* tiles;
+    uint32_t coefs, levels, words, groups, atoms, splits, item_tiles, tile_items;
+};
+
+// 16 slots from slot s of the row of `digits` per coefficient, as bytes
+template <int BITS, class Digit>
+__device__ __forceinline__ uint4 one_hot16(uint32_t s, Digit digit) {
+    uint64_t lo = 0, hi = 0;
+    auto set = [&](uint32_t pos) {  // pos >= 16: outside this chunk
+        const uint64_t bit = 1ull << (8 * (pos & 7u));
+        lo |= pos < 8 ? bit : 0ull;
+        hi |= (pos >> 3) == 1 ? bit : 0ull;
+    };
+    if constexpr (BITS <= 4) {
+#pragma unroll
+        for (uint32_t d = 0; d < (16u >> BITS); ++d) set((d << BITS) + digit((s >> BITS) + d));
+    } else {
+        set(digit(s >> BITS) - (s & ((1u << BITS) - 1u)));
+    }
+    return make_uint4(static_cast<uint32_t>(lo), static_cast<uint32_t>(lo >> 32), static_cast<uint32_t>(hi),
+                      static_cast<uint32_t>(hi >> 32));
+}
+
+template <class Src, int BITS, int PLANES>
+__global__ void __launch_bounds__(kThreads, 1) k_ks_mma(const Src src, const KsGrid g) {
+    extern __shared__ uint8_t raw_smem[];
+    const uint32_t pad = (1024u - (smem_u32(raw_smem) & 1023u)) & 1023u;
+    uint8_t* smem = raw_smem + pad;
+    uint8_t* key_ring = smem;
+    using Cfg = KsCfg<PLANES>;
+    constexpr uint32_t KEYS = Cfg::KEY_STAGES, ITEMS = Cfg::ITEMS;
+    uint8_t* hot_ring = smem + Cfg::hot_off;
+    uint32_t** ptrs = reinterpret_cast<uint32_t**>(smem + Cfg::ptr_off);  // [ITEMS][2]
+    uint64_t* key_full = reinterpret_cast<uint64_t*>(smem + Cfg::bar_off);
+    uint64_t* key_empty = key_full + KEYS;
+    uint64_t* hot_full = key_empty + KEYS;
+    uint64_t* hot_empty = hot_full + kHotStages;
+    uint64_t* done = hot_empty + kHotStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    uint32_t id = blockIdx.x;
+    const uint32_t tile = id % g.item_tiles;
+    id /= g.item_tiles;
+    const uint32_t split = id % g.splits;
+    id /= g.splits;
+    const uint32_t group = id % g.groups, fn = id / g.groups;
+    const uint32_t item0 = tile * g.tile_items;
+    const uint32_t live = min(g.tile_items, src.items - item0), n = (live + 15u) & ~15u;
+    const uint32_t atom0 = static_cast<uint32_t>(static_cast<uint64_t>(g.atoms) * split / g.splits);
+    const uint32_t atom1 = static_cast<uint32_t>(static_cast<uint64_t>(g.atoms) * (split + 1) / g.splits);
+    const uint32_t steps = atom1 - atom0;
+
+    if (tid == 0) {
+        for (uint32_t i = 0; i < KEYS; ++i) {
+            mbar_init(key_full + i, 1);
+            mbar_init(key_empty + i, 1);
+        }
+        for (uint32_t i = 0; i < kHotStages; ++i) {
+            mbar_init(hot_full + i, kGenWarps);
+            mbar_init(hot_empty + i, 1);
+        }
+        mbar_init(done, 1);
+        *abort_flag = 0;
+        mbar_init_fence();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, 512);
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (mbar_wait_bounded(bar, parity, kWaitLimit)) return true;
+        *abort_flag = 1;
+        return false;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {  // stream the key tiles
+            const uint8_t* from = g.tiles + ((static_cast<size_t>(fn) * g.groups + group) * g.atoms + atom0) *
+                                                (static_cast<size_t>(PLANES) * kTile);
+            const uint32_t total = steps * PLANES;
+            uint32_t issued = 0;
+            for (; issued < total && !*abort_flag; ++issued) {
+                const uint32_t st = issued % KEYS, use = issued / KEYS;
+                if (use && !wait(key_empty + st, (use - 1) & 1u)) break;
+                mbar_arrive_expect_tx(key_full + st, kTile);
+                bulk_load(key_ring + st * kTile, from + static_cast<size_t>(issued) * kTile, kTile, key_full + st);
+            }
+            if (*abort_flag) {  // the copies in flight land before the CTA may leave
+                for (uint32_t i = issued > KEYS ? issued - KEYS : 0; i < issued; ++i)
+                    mbar_wait_bounded(key_full + i % KEYS, (i / KEYS) & 1u, kWaitLimit);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {  // issue the products
+            const uint32_t idesc = i8_idesc(n);
+            bool ok = true;
+            for (uint32_t a = 0; a < steps && ok; ++a) {
+                const uint32_t hs = a % kHotStages;
+                ok = wait(hot_full + hs, (a / kHotStages) & 1u);
+                const uint64_t hot = tile_desc(smem_u32(hot_ring + hs * Cfg::HOT));
+                for (uint32_t p = 0; p < PLANES && ok; ++p) {
+                    const uint32_t t = a * PLANES + p, st = t % KEYS;
+                    ok = wait(key_full + st, (t / KEYS) & 1u);
+                    if (!ok || *abort_flag) {
+                        ok = false;
+                        break;
+                    }
+                    tmem_fence_after();
+                    const uint64_t key = tile_desc(smem_u32(key_ring + st * kTile));
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)  // 32 slots per instruction
+                        mma_i8(tmem + p * ITEMS, key + 2 * k, hot + 2 * k, idesc, (a | k) != 0);
+                    mma_commit(key_empty + st);
+                }
+                if (ok) mma_commit(hot_empty + hs);
+            }
+            mma_commit(done);
+        }
+    } else {
+        // one-hot rows: thread -> PART consecutive slots of one item's row
+        constexpr uint32_t PART = ITEMS == 256 ? 128 : 64;
+        const uint32_t gt = tid - 64, row = gt % ITEMS, s_off = (gt / ITEMS) * PART;
+        const bool mine = row < live;
+        typename Src::Row r{};
+        if (mine) {
+            r = src.row(item0 + row);
+            if (s_off == 0) src.rows(item0 + row, fn, g.words, ptrs[2 * row], ptrs[2 * row + 1]);
+        }
+        auto load = [&](uint32_t i) { return mine && i < g.coefs ? src.word(r, i) : 0u; };
+        // the first two coefficients of a part are loaded one step ahead
+        auto first_of = [&](uint32_t a) { return ((((atom0 + a) * 128 + s_off) >> BITS) / g.levels); };
+        uint32_t i0 = first_of(0), n0 = load(i0), n1 = load(i0 + 1);
+        for (uint32_t a = 0; a < steps; ++a) {
+            const uint32_t hs = a % kHotStages, use = a / kHotStages;
+            const uint32_t x0 = n0, x1 = n1, base_i = i0;
+            if (a + 1 < steps) {
+                const uint32_t ni = first_of(a + 1);
+                if (ni != i0) {
+                    i0 = ni;
+                    n0 = load(i0);
+                    n1 = load(i0 + 1);
+                }
+            }
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+            if (use && !__all_sync(0xffffffffu, wait(hot_empty + hs, (use - 1) & 1u))) break;
+            if (row < n) {
+                uint8_t* dst = hot_ring + hs * Cfg::HOT + row * 128;
+                const uint32_t s0 = (atom0 + a) * 128 + s_off;
+                uint32_t t_at = s0 >> BITS, i = base_i, l = t_at - base_i * g.levels, x = x0;
+                auto digit = [&](uint32_t t) {  // called for t_at, then ascending by at most one
+                    if (t != t_at) {
+                        t_at = t;
+                        if (++l == g.levels) {
+                            l = 0;
+                            ++i;
+                            x = i == base_i + 1 ? x1 : load(i);
+                        }
+                    }
+                    return (x >> (32 - (l + 1) * BITS)) & ((1u << BITS) - 1u);
+                };
+#pragma unroll
+                for (uint32_t c = 0; c < PART / 16; ++c) {
+                    const uint32_t chunk = s_off / 16 + c;
+                    *reinterpret_cast<uint4*>(dst + ((chunk ^ (row & 7u)) << 4)) = one_hot16<BITS>(s0 + 16 * c, digit);
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(hot_full + hs);
+        }
+        // this range's sums: lane = output word, column p * ITEMS + item
+        const bool ok = __all_sync(0xffffffffu, wait(done, 0) && !*abort_flag);
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kGenWarps) : "memory");  // ptrs
+        tmem_fence_after();
+        const uint32_t word = group * 128 + (warp & 3u) * 32 + lane;
+        // two warps per lane quadrant take alternate blocks of 16 items
+        for (uint32_t c0 = 16 * ((warp - 2) >> 2); c0 < n && ok; c0 += 32) {
+            uint32_t sum[16];
+#pragma unroll
+            for (int p = 0; p < PLANES; ++p) {
+                uint32_t v[16];
+                tmem_load16(tmem_quadrant_addr(tmem, p * ITEMS + c0), v);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) sum[q] = p ? sum[q] + (v[q] << (8 * p)) : v[q];
+            }
+            if (word < g.words) {
+#pragma unroll
+                for (uint32_t q = 0; q < 16; ++q) {
+                    if (c0 + q >= live) break;
+                    uint32_t* dst = word + 1 < g.words ? ptrs[2 * (c0 + q)] + static_cast<size_t>(word) * Src::kStep
+                                                       : ptrs[2 * (c0 + q) + 1];
+                    atomicAdd(dst, Src::kSubtract ? 0u - sum[q] : sum[q]);
+                }
+            }
+        }
+        tmem_fence_before();
+    }
+    __syncthreads();
+    tmem_fence_after();
+    if (tid == 0 && *abort_flag) atomicOr(&g_ks_fault, 1u);
+    if (warp == 1) {
+        __syncwarp();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+// outputs of the gate switch before the sums: 0 and the extracted b
+__global__ void __launch_bounds__(256) k_ks_gate_init(const GateSrc src, uint32_t words) {
+    uint32_t *a, *last;
+    src.rows(blockIdx.x, 0, words, a, last);
+    for (uint32_t w = threadIdx.x; w + 1 < words; w += blockDim.x) a[w] = 0u;
+    if (threadIdx.x == 0) *last = __ldg(src.ext + static_cast<size_t>(blockIdx.x) * (src.coefs + 1) + src.coefs);
+}
+
+__global__ void __launch_bounds__(256) k_ks_extract_init(const ExtractArgs e) {
+    const uint32_t t = blockIdx.x;
+    for (uint32_t k = threadIdx.x; k < e.n; k += blockDim.x) e.out_a[static_cast<size_t>(t) * e.out_stride + k] = 0;
+    if (threadIdx.x == 0) {
+        const uint32_t info = __ldg(e.info + t);
+        const uint64_t bv = e.words[(static_cast<size_t>(info >> 16) * 2 + 1) * e.N + (info & 0xffffu)];
+        e.out_b[t] = extract_ms_pow2(bv, e.q_over_Q, e.mask);
+    }
+}
+
+// the sums (low words, mod 2^32) mod qKS, then qKS -> q
+__global__ void __launch_bounds__(256) k_ks_extract_finish(const ExtractArgs e) {
+    const uint32_t t = blockIdx.x;
+    for (uint32_t k = threadIdx.x; k <= e.n; k += blockDim.x) {
+        uint64_t* p = k < e.n ? e.out_a + static_cast<size_t>(t) * e.out_stride + k : e.out_b + t;
+        *p = extract_qks_to_q(static_cast<uint32_t>(*p) & e.mask, e.scale, e.qks, e.q_lwe);
+    }
+}
+
+// one 16 KB tile set (all planes) of a (function, group, step) per CTA: thread -> 16-slot chunks
+template <class Word>
+__device__ __forceinline__ void build_tile(const KsShape& k, uint8_t* tiles, Word word_at) {
+    const uint32_t atoms = gridDim.x, atom = blockIdx.x, group = blockIdx.y, fn = blockIdx.z;
+    const uint32_t slots = k.coefs * k.levels << k.bits, vmask = (1u << k.bits) - 1u;
+    uint8_t* base = tiles + ((static_cast<size_t>(fn) * gridDim.y + group) * atoms + atom) *
+                                (static_cast<size_t>(k.planes) * kTile);
+    for (uint32_t c = threadIdx.x / 128; c < 8; c += blockDim.x / 128) {
+        const uint32_t r = threadIdx.x % 128, w = group * 128 + r;
+        uint32_t plane[4][4] = {};
+        for (uint32_t q = 0; q < 16; ++q) {
+            const uint32_t s = atom * 128 + 16 * c + q;
+            uint32_t v = 0;
+            if (w < k.words && s < slots) {
+                const uint32_t t = s >> k.bits, i = t / k.levels;
+                v = word_at(fn, i, t - i * k.levels, s & vmask, w);
+            }
+#pragma unroll
+            for (uint32_t p = 0; p < 4; ++p) plane[p][q >> 2] |= ((v >> (8 * p)) & 0xffu) << (8 * (q & 3u));
+        }
+#pragma unroll
+        for (uint32_t p = 0; p < 4; ++p)
+            if (p < k.planes)
+                *reinterpret_cast<uint4*>(base + static_cast<size_t>(p) * kTile + r * 128 + ((c ^ (r & 7u)) << 4)) =
+                    make_uint4(plane[p][0], plane[p][1], plane[p][2], plane[p][3]);
+    }
+}
+
+__global__ void __launch_bounds__(512) k_ks_build(const KsShape k, const uint32_t* key, uint32_t rows_per_digit,
+                                                  uint32_t row_stride, uint8_t* tiles) {
+    const uint32_t skip = (1u << k.bits) - rows_per_digit;  // 1: no stored row for digit value 0
+    build_tile(k, tiles, [&](uint32_t fn, uint32_t i, uint32_t l, uint32_t v, uint32_t w) -> uint32_t {
+        if (v < skip) return 0u;
+        const size_t row = ((static_cast<size_t>(fn) * k.coefs + i) * k.levels + l) * rows_per_digit + v - skip;
+        return __ldg(key + row * row_stride + w);
+    });
+}
+
+__global__ void __launch_bounds__(512) k_ks_build_u16(const KsShape k, const uint16_t* key, uint32_t row_stride,
+                                                      uint8_t* tiles) {
+    build_tile(k, tiles, [&](uint32_t, uint32_t i, uint32_t l, uint32_t v, uint32_t w) -> uint32_t {
+        const size_t row = ((static_cast<size_t>(l) * k.coefs + i) << k.bits) + v;
+        return __ldg(key + row * row_stride + w);
+    });
+}
+
+// Items in equal tiles (a multiple of 16, at most the column block); the slots in `splits` ranges such that
+// the CTAs fill the SMs: the split that minimises waves x (steps of a range + a fixed cost of
+// about 6 steps for start, drain and the adds), counted in 128-slot steps.
+KsGrid make_grid(const KsShape& k, const uint8_t* tiles, uint32_t items, uint32_t sms) {
+    KsGrid g{};
+    g.tiles = tiles;
+    g.coefs = k.coefs;
+    g.levels = k.levels;
+    g.words = k.words;
+    g.groups = k.groups();
+    g.atoms = k.atoms();
+    const uint32_t most = 512 / k.planes, tiles_n = (items + most - 1) / most;
+    g.tile_items = ((items + tiles_n - 1) / tiles_n + 15) & ~15u;
+    g.item_tiles = (items + g.tile_items - 1) / g.tile_items;
+    const uint64_t units = static_cast<uint64_t>(k.funcs) * g.groups * g.item_tiles;
+    uint64_t best = ~0ull;
+    g.splits = 1;
+    for (uint32_t s = 1; s <= g.atoms && s <= 256; ++s) {
+        const uint64_t cost = ((units * s + sms - 1) / sms) * ((g.atoms + s - 1) / s + 6);
+        if (cost < best) {
+            best = cost;
+            g.splits = s;
+        }
+    }
+    return g;
+}
+
+template <class Src, int BITS, int PLANES>
+cudaError_t launch(const KsShape& k, const uint8_t* tiles, const Src& src, cudaStream_t s) {
+    static bool configured[64] = {};  // per device
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if (!configured[dev]) {
+        e = cudaFuncSetAttribute(k_ks_mma<Src, BITS, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(KsCfg<PLANES>::bytes));
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    const KsGrid g = make_grid(k, tiles, src.items, static_cast<uint32_t>(sms));
+    const uint64_t ctas = static_cast<uint64_t>(k.funcs) * g.groups * g.splits * g.item_tiles;
+    if (ctas > 0x7fffffffull) return cudaErrorInvalidValue;
+    k_ks_mma<Src, BITS, PLANES><<<static_cast<unsigned>(ctas), kThreads, KsCfg<PLANES>::bytes, s>>>(src, g);
+    return cudaGetLastError();
+}
+
+template <class Src, int PLANES>
+cudaError_t launch_bits(const KsShape& k, const uint8_t* tiles, const Src& src, cudaStream_t s) {
+    switch (k.bits) {
+        case 1: return launch<Src, 1, PLANES>(k, tiles, src, s);
+        case 2: return launch<Src, 2, PLANES>(k, tiles, src, s);
+        case 3: return launch<Src, 3, PLANES>(k, tiles, src, s);
+        case 4: return launch<Src, 4, PLANES>(k, tiles, src, s);
+        case 5: return launch<Src, 5, PLANES>(k, tiles, src, s);
+        case 6: return launch<Src, 6, PLANES>(k, tiles, src, s);
+        case 7: return launch<Src, 7, PLANES>(k, tiles, src, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace
+
+cudaError_t ks_build_tiles(const KsShape& k, const uint32_t* key, uint32_t rows_per_digit, uint32_t row_stride,
+                           uint8_t* tiles, cudaStream_t s) {
+    k_ks_build<<<dim3(k.atoms(), k.groups(), k.funcs), 512, 0, s>>>(k, key, rows_per_digit, row_stride, tiles);
+    return cudaGetLastError();
+}
+
+cudaError_t ks_build_tiles_u16(const KsShape& k, const uint16_t* key, uint32_t row_stride, uint8_t* tiles,
+                               cudaStream_t s) {
+    k_ks_build_u16<<<dim3(k.atoms(), k.groups(), k.funcs), 512, 0, s>>>(k, key, row_stride, tiles);
+    return cudaGetLastError();
+}
+
+cudaError_t ks_mma_gate(const KsShape& k, const uint8_t* tiles, const uint32_t* ext, uint32_t items, uint32_t round,
+                        uint32_t* out_a, uint32_t* out_b, const GateReq* reqs, uint32_t num_reqs, cudaStream_t s) {
+    if (items == 0) return cudaSuccess;
+    const GateSrc src{ext, k.coefs, items, round, out_a, out_b, reqs, num_reqs};
+    k_ks_gate_init<<<items, 256, 0, s>>>(src, k.words);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_bits<GateSrc, 4>(k, tiles, src, s);
+}
+
+cudaError_t ks_mma_tcb(const KsShape& k, const uint8_t* tiles, const uint64_t* ext, uint32_t items, uint32_t* rgsw,
+                       cudaStream_t s) {
+    if (items == 0) return cudaSuccess;
+    const TcbSrc src{ext, k.coefs, items, k.funcs, rgsw};
+    cudaError_t e = cudaMemsetAsync(rgsw, 0, static_cast<size_t>(items) * k.funcs * k.words * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    switch (k.bits) {  // base_bits * levels = 32
+        case 1: return launch<TcbSrc, 1, 4>(k, tiles, src, s);
+        case 2: return launch<TcbSrc, 2, 4>(k, tiles, src, s);
+        case 4: return launch<TcbSrc, 4, 4>(k, tiles, src, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t ks_mma_extract(const KsShape& k, const uint8_t* tiles, const ExtractArgs& a, uint32_t count,
+                           cudaStream_t s) {
+    if (count == 0) return cudaSuccess;
+    const ExtractSrc src{a, count};
+    k_ks_extract_init<<<count, 256, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    e = launch_bits<ExtractSrc, 2>(k, tiles, src, s);
+    if (e != cudaSuccess) return e;
+    k_ks_extract_finish<<<count, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t ks_mma_fault(uint32_t* out, bool clear) {
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(out, g_ks_fault, sizeof(uint32_t));
+    const uint32_t zero = 0;
+    if (e == cudaSuccess && clear && *out) e = cudaMemcpyToSymbol(g_ks_fault, &zero, sizeof(uint32_t));
+    return e;
+}
+
+}  // namespace cbs

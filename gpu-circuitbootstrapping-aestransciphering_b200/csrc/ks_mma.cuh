@@ -1,0 +1,52 @@
+// ks_mma.cuh -- LWE / private functional key switching as an integer matrix product on the
+// tensor cores (ks_mma.cu): launch interface.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+#include "torus.cuh"
+
+namespace cbs {
+
+// The shape of one key: `funcs` independent keys, each with `coefs` input coefficients of
+// `levels` digits of `bits` bits, and rows of `words` output words of `planes` bytes.
+struct KsShape {
+    uint32_t funcs, coefs, levels, bits, words, planes;
+    uint32_t groups() const { return (words + 127) / 128; }                  // 128-word groups
+    uint32_t atoms() const { return ((coefs * levels << bits) + 127) / 128; }  // 128-slot steps
+    size_t tile_bytes() const { return static_cast<size_t>(funcs) * groups() * atoms() * planes * (128 * 128); }
+};
+
+// key rows [funcs][coefs][levels][rows_per_digit][row_stride] (u32 or u16 words; rows_per_digit =
+// 2^bits, or 2^bits - 1 without the all-zero row of digit value 0) -> byte-plane tiles
+cudaError_t ks_build_tiles(const KsShape& k, const uint32_t* key, uint32_t rows_per_digit, uint32_t row_stride,
+                           uint8_t* tiles, cudaStream_t s);
+// the same from the u16 layout [levels][coefs][2^bits][row_stride]
+cudaError_t ks_build_tiles_u16(const KsShape& k, const uint16_t* key, uint32_t row_stride, uint8_t* tiles,
+                               cudaStream_t s);
+
+// Digit widths that take the matrix form: up to 7 bits.  A digit costs 2^bits slots here and one
+// row in the gather, so the gain shrinks with the width.  Gate switch of 592 ciphertexts (n = 636,
+// N = 1024): 2 x 8 bits 3024 -> 84 us, 5 x 3 bits 1981 -> 170 us, 7 x 2 bits 1674 -> 421 us (64
+// ciphertexts: 1134 -> 25 us at 2 bits, 861 -> 25-45 us at 7); each further bit doubles the product
+// and not the gather, and a batch of a few thousand would lose at 8 bits.
+inline bool ks_mma_bits(uint32_t bits) { return bits >= 1 && bits <= 7; }
+
+// gate key switch N -> n of `items` extracted ciphertexts ext [items][N + 1] (b last), digits of
+// ext + round; outputs as k_gate_keyswitch (out_a / out_b, or the requests' buffers)
+cudaError_t ks_mma_gate(const KsShape& k, const uint8_t* tiles, const uint32_t* ext, uint32_t items, uint32_t round,
+                        uint32_t* out_a, uint32_t* out_b, const GateReq* reqs, uint32_t num_reqs, cudaStream_t s);
+// PFKS of `items` level-2 ciphertexts ext [items][coefs] into rgsw [items][funcs][words]
+cudaError_t ks_mma_tcb(const KsShape& k, const uint8_t* tiles, const uint64_t* ext, uint32_t items, uint32_t* rgsw,
+                       cudaStream_t s);
+struct ExtractArgs;
+// sample extraction + key switch of k_extract_keyswitch
+cudaError_t ks_mma_extract(const KsShape& k, const uint8_t* tiles, const ExtractArgs& a, uint32_t count,
+                           cudaStream_t s);
+// device fault word: nonzero when a bounded wait of these kernels ran out
+cudaError_t ks_mma_fault(uint32_t* out, bool clear);
+
+}  // namespace cbs

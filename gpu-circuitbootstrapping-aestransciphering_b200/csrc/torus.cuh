@@ -56,8 +56,6 @@ struct GateArgs {
 
 cudaError_t gate_blind_rotate(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);    // 32-bit torus
 cudaError_t gate_blind_rotate64(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);  // 64-bit torus
-cudaError_t gate_keyswitch(const GateArgs& a, const uint32_t* ksk, uint32_t n, uint32_t N, uint32_t ks_bits,
-                           uint32_t ks_levels, uint32_t* out_a, uint32_t* out_b, cudaStream_t s);
 
 uint32_t torus_from_double(double x);
 uint32_t torus_noise(Rng& rng, double sigma);

@@ -663,6 +663,12 @@ cbs_status cbs_tcb_encrypt_bits(const cbs_tcb_context *ctx, const uint8_t *h_bit
 cbs_status cbs_tcb_circuit_bootstrap_device(cbs_tcb_context *ctx, const uint32_t *d_a, const uint32_t *d_b,
                                             uint32_t count, uint64_t *d_ext, uint32_t *d_rgsw, cbs_stream_t stream);
 
+/* Device fault word of the tensor-core key switches (gate, PFKS and extraction) of the current
+ * device: nonzero when a bounded wait inside one of them ran out (about a second); that launch
+ * then finished with unreliable outputs instead of hanging.  Synchronizes the device; clear != 0
+ * resets the word.  0 after correct runs.  No reference counterpart. */
+cbs_status cbs_keyswitch_device_fault(uint32_t *out, int clear);
+
 /* ------------------------------------------------------------------------------------
  * RNS (Phantom) core: multi-prime NTT and hybrid key switching, CKKS form.
  * Key modulus chain = the size_q primes of Q followed by the size_p special primes P
