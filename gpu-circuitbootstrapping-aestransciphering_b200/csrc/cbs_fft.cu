@@ -573,32 +573,36 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
 }
 
 // Paired form of the two-digit grouped blind rotation (mb = 2, 2^18 x 2 gadget): two
-// ciphertexts per CTA of 512 threads, so an SM holds 16 warps instead of 8.  To fit 128
-// registers and the shared memory of two ciphertexts, the work per group is split by output
-// column instead of by input polynomial:
-//  1. each half (128 threads) transforms the two digits of its polynomial in lockstep, with the
-//     digits read straight from the accumulator (no digit buffer), and stores both spectra;
-//  2. after a CTA barrier, the 512 threads split by output column, slot half and position: each
-//     forms its 4 slots of output column mh for BOTH ciphertexts from all four digit spectra of
-//     each, y_mh += x_row (sum_S m_S(psi) K_S[row][mh]) over the rows, so every key word loaded
-//     feeds two ciphertexts; c_i(psi) = zeta^(a_i e_t) omega8^k - 1 is recomputed per slot;
-//  3. after a second barrier (every spectrum read) the outputs go to the [mh][0] spectrum
-//     buffers, and after a third, half h of each ciphertext inverse-transforms its column and
-//     adds the rounded result into the accumulator positions it owns.
-// The accumulator lives in tensor memory: a thread's transform reads and writes the same 16
-// coefficients every group (positions e, e + M of its 8 slots), so they stay in its TMEM lane
-// (ht, the same lane its warp quadrant reaches), 32 columns per half and ciphertext, 128 in all.
-// Shared memory: the FFT tables once, then per ciphertext the spectra [2 halves][2 digits][N/2]
-// (146 KB at N = 2048); the final accumulator passes through the spectra area for the MV
-// split.  An odd batch's last CTA runs its second ciphertext as a copy of the first and writes
-// nothing for it.
+// ciphertexts per CTA of 512 threads, so an SM holds 16 warps and every key word loaded feeds
+// two ciphertexts.  Thread ht of each 128-thread half (ciphertext, polynomial) transforms the two
+// digits of its polynomial in lockstep and ends with slots 8 ht .. 8 ht + 7; everything that
+// passes between the phases of a group stays in its lane, so it goes through tensor memory
+// (TMEM) and not through shared memory, which the transforms' exchanges keep busy:
+//  * the accumulator: the transform reads and writes the same 16 coefficients every group
+//    (positions e, e + M of its 8 slots), 32 columns per half;
+//  * the digit spectra, 32 columns per slot: [row][ciphertext];
+//  * the outputs, 32 columns per (ciphertext, column).
+// TMEM lane = ht, and a warp reaches the lanes of its quadrant only, which are the same lanes in
+// the four halves: the four warps of a quadrant exchange spectra and outputs among themselves,
+// so the two barriers around the product phase join 128 threads, not the CTA.
+// Per group: 1. digit transforms, spectra to TMEM; 2. warp g of a quadrant forms slots 2g and
+// 2g + 1 of both output columns of both ciphertexts: per column and subset S the sums
+// sum_row x_row K_S[row], each key word loaded once (six in flight per thread: the phase is bound
+// by the latency of these loads), then sum_S m_S(psi) over the three sums (c_0 (S_0 + c_1 S_01) +
+// c_1 S_1, c_i(psi) = psi^(a_i) - 1); 3. each half
+// inverse-transforms its column and adds the rounded result into its accumulator.
+// An odd batch's last CTA runs its second ciphertext as a copy of the first and writes nothing
+// for it.
+// Measured at 296 ciphertexts (one wave, N = 2048, n = 630): 4.90 -> 3.83 ms (16.5 -> 12.9 us per
+// bootstrap) against spectra and outputs in shared memory, each thread forming one column from
+// three key loads at a time (62 % of the data-pipe cycles, the product phase waiting on L2).
 template <int LOGN>
 __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     k_blind_rotate_fft_mb2_x2(const BlindRotateArgs a, const FftKeyArgs f, uint32_t batch) {
     constexpr int LOGM = LOGN - 1;
     constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, TWO_N = 2 * N;
     constexpr uint32_t KS = 3, DIGITS = 2, L2 = 2 * DIGITS;
-    constexpr uint32_t TMEM_COLS = 128;  // 4 (ciphertext, half) pairs x 32 columns
+    constexpr uint32_t TMEM_COLS = 512, SPEC_COL = 128, OUT_COL = 384;
     static_assert(TH == 128, "one TMEM lane per transform thread");
     using Tb = FftTab<LOGM>;
     extern __shared__ __align__(16) uint64_t smem[];
@@ -608,7 +612,7 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     const uint32_t ct_raw = 2 * blockIdx.x + c2;
     const bool live = ct_raw < batch;
     const uint32_t ct = live ? ct_raw : batch - 1;
-    // after the tables: the TMEM base address (16 bytes), then per ciphertext spec [2][2][M]
+    // after the tables: the TMEM base address (16 bytes), then per ciphertext exchange [2][2][M]
     constexpr size_t tab_words = (Tb::size() * sizeof(double2) + 15) / 16 * 2;  // 16-byte aligned, in u64
     constexpr size_t ct_words = 4 * M * 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + tab_words);
@@ -668,10 +672,18 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     }
     __syncthreads();
 
-    // named barriers: 1 + c2 over the ciphertext's 256 threads, 3 + 2 c2 + h over a half
-    const uint32_t ct_bar = 1 + c2, half_id = 3 + 2 * c2 + h;
+    // named barriers: 1 + c2 over the ciphertext's 256 threads, 3 + 2 c2 + h over a half, 7 + q over
+    // the four warps of TMEM lane quadrant q
+    const uint32_t ct_bar = 1 + c2, half_id = 3 + 2 * c2 + h, quad_id = 7 + ht / 32;
     auto ct_sync = [ct_bar]() { asm volatile("bar.sync %0, %1;" ::"r"(ct_bar), "n"(2 * TH) : "memory"); };
     auto half_bar = [half_id]() { asm volatile("bar.sync %0, %1;" ::"r"(half_id), "n"(TH) : "memory"); };
+    // this thread's TMEM stores are visible to the quadrant's warps after it
+    auto quad_sync = [quad_id]() {
+        tmem_wait_store();
+        tmem_fence_before();
+        asm volatile("bar.sync %0, %1;" ::"r"(quad_id), "n"(128) : "memory");
+        tmem_fence_after();
+    };
     const DigitBias bias(1u << (gbits - 1));
     const uint32_t fmask = (1u << gbits) - 1u;
     const uint64_t* arow[2];
@@ -680,17 +692,14 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
         const uint32_t cr = 2 * blockIdx.x + c;
         arow[c] = a.a + static_cast<size_t>(cr < batch ? cr : batch - 1) * a.a_stride;
     }
-    // the product phase's split of the 512 threads: output column mh, slot half sh, position mt
-    const uint32_t mh = tid / (2 * TH), sh = (tid / TH) & 1u, mt = tid % TH;
-    auto spec_of = [&](int c) {
-        return reinterpret_cast<double2*>(smem + tab_words + 2 + c * ct_words);
-    };
+    const uint32_t pg = tid / TH;  // product phase: slots 2 pg and 2 pg + 1 of lane ht
+    const uint32_t tspec = tmem_quadrant_addr(tmem_base, SPEC_COL), tout = tmem_quadrant_addr(tmem_base, OUT_COL);
     const uint32_t groups = (a.n + 1) / 2;
     constexpr size_t kstride = static_cast<size_t>(L2) * 2 * M;  // spectra between subsets of a group
     for (uint32_t g = 0; g < groups; ++g) {
         // 1. the two digit transforms of polynomial h, digits read from the accumulator
-        double2 x0[8], x1[8];
         {
+            double2 x0[8], x1[8];
             uint32_t wa[16], wb[16];
             tmem_load16(tacc, wa);
             tmem_load16(tacc + 16, wb);
@@ -703,70 +712,75 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
             fft_forward2_to_regs<LOGM>(
                 my_s0, my_s1, ht, tab, [&](int j, uint32_t) { return digit_pair(j, 0); },
                 [&](int j, uint32_t) { return digit_pair(j, gbits); }, x0, x1, half_bar);
-        }
-        half_bar();  // the transforms' last reads of my_s0 / my_s1 are done
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            my_s0[cswz(8 * ht + j)] = x0[j];
-            my_s1[cswz(8 * ht + j)] = x1[j];
+            for (int j = 0; j < 8; ++j) {  // rows h and 2 + h of slot j
+                tmem_store_complex(tspec + 32 * j + 8 * h + 4 * c2, x0[j]);
+                tmem_store_complex(tspec + 32 * j + 8 * (2 + h) + 4 * c2, x1[j]);
+            }
         }
-        // the group's rotations of both ciphertexts (read before the barrier)
+        // the group's rotations of both ciphertexts (before the barrier)
         const uint32_t idx0 = 2 * g, idx1 = idx0 + 1;
         uint32_t at[2][2];
-        double2 ub[2][2];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             at[c][0] = special_ms_f(__ldg(arow[c] + idx0), TWO_N, a.q_lwe, a.bitwidth);
             at[c][1] = idx1 < a.n ? special_ms_f(__ldg(arow[c] + idx1), TWO_N, a.q_lwe, a.bitwidth) : 0u;
-            ub[c][0] = zeta_pow<LOGN>(tws, mult_base<LOGN>(mt, at[c][0]));
-            ub[c][1] = zeta_pow<LOGN>(tws, mult_base<LOGN>(mt, at[c][1]));
         }
-        __syncthreads();
-        // 2. output column mh, slots 4 sh .. 4 sh + 3, of both ciphertexts: each key word feeds
-        // both, through the combined key sum_S m_S(psi) K_S[row][mh] of each
-        const double2* gk = f.bskf + static_cast<size_t>(g) * KS * kstride + static_cast<size_t>(mh) * M + mt;
-        double2 y[2][4];
+        quad_sync();
+        // 2. slots 2 pg, 2 pg + 1 of both columns of both ciphertexts
+        const double2* gk = f.bskf + static_cast<size_t>(g) * KS * kstride + ht;
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const uint32_t j = 4 * sh + jj;
-            const uint32_t r3 = ((j & 1) << 2) | (j & 2) | ((j >> 2) & 1);
-            double2 cc[2][3];
+        for (int jj = 0; jj < 2; ++jj) {
+            const uint32_t j = 2 * pg + jj;
+            const double2* kj = gk + j * TH;
+            double2 s[2][2][KS];  // [column][ciphertext][subset]
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (uint32_t row = 0; row < L2; ++row) {  // row 2d + p: digit d of polynomial p
+                double2 k[2][KS];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    cc[c][i] = cmul(ub[c][i], omega8<double2>((at[c][i] * r3) & 7u));
-                    cc[c][i].x -= 1.0;
-                }
-                cc[c][2] = cmul(cc[c][0], cc[c][1]);
-                y[c][jj] = make_double2(0.0, 0.0);
-            }
-            const uint32_t xs = cswz(8 * mt + j);
+                for (int col = 0; col < 2; ++col)
 #pragma unroll
-            for (uint32_t row = 0; row < L2; ++row) {
-                // row 2d + p: digit d of polynomial p, spectrum buffer [p][d]
-                const double2* kr = gk + static_cast<size_t>(row) * 2 * M + j * TH;
-                const double2 k0 = __ldg(kr), k1 = __ldg(kr + kstride), k2 = __ldg(kr + 2 * kstride);
-                const uint32_t xo = ((row & 1u) * 2 + (row >> 1)) * M + xs;
+                    for (uint32_t q = 0; q < KS; ++q)
+                        k[col][q] = __ldg(kj + q * kstride + static_cast<size_t>(row * 2 + col) * M);
+                uint32_t xw[8];
+                tmem_load8(tspec + 32 * j + 8 * row, xw);
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    double2 kc = cmul(cc[c][0], k0);
-                    cfma(kc, cc[c][1], k1);
-                    cfma(kc, cc[c][2], k2);
-                    cfma(y[c][jj], spec_of(c)[xo], kc);
+                    const double2 x = tmem_complex(xw, c);
+#pragma unroll
+                    for (int col = 0; col < 2; ++col)
+#pragma unroll
+                        for (uint32_t q = 0; q < KS; ++q) {
+                            if (row == 0) s[col][c][q] = cmul(x, k[col][q]);
+                            else cfma(s[col][c][q], x, k[col][q]);
+                        }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                double2 cc[2];  // c_i(psi) of this slot
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    cc[i] = zeta_pow<LOGN>(tws, slot_exp<LOGN>(mult_base<LOGN>(ht, at[c][i]), at[c][i], j));
+                    cc[i].x -= 1.0;
+                }
+#pragma unroll
+                for (int col = 0; col < 2; ++col) {
+                    cfma(s[col][c][0], cc[1], s[col][c][2]);
+                    double2 v = cmul(cc[0], s[col][c][0]);
+                    cfma(v, cc[1], s[col][c][1]);
+                    tmem_store_complex(tout + 32 * (2 * c + col) + 4 * j, v);
                 }
             }
         }
-        __syncthreads();  // every spectrum read is done: the outputs take the [mh][0] buffers
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) spec_of(c)[(2 * mh) * M + cswz(8 * mt + 4 * sh + jj)] = y[c][jj];
-        __syncthreads();
+        quad_sync();
         double2 yv[8];
+        {
+            uint32_t w[32];
+            tmem_load32(tout + 32 * (2 * c2 + h), w);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) yv[j] = my_s0[cswz(8 * ht + j)];
-        half_bar();  // every output slot is in registers before the transform reuses the buffer
+            for (int j = 0; j < 8; ++j) yv[j] = tmem_complex(w, j);
+        }
         // 3. inverse transform, rounding, accumulate into the TMEM accumulator (each 16-column
         // half read when its first slot arrives, written back after its last)
         uint32_t wacc[16];
