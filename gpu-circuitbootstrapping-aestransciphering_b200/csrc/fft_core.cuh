@@ -307,6 +307,47 @@ constexpr bool inv_exchange_in_warp(int p) {
     return ((1u << LOGM) >> (3 * p)) / 8 <= 32;
 }
 
+template <class C>
+__device__ __forceinline__ C shfl_pair(C v) {
+    C r;
+    r.x = __shfl_xor_sync(0xffffffffu, v.x, 1);
+    r.y = __shfl_xor_sync(0xffffffffu, v.y, 1);
+    return r;
+}
+// The exchange before a one-stage forward tail: threads 2k and 2k + 1 hold the even and the odd
+// elements of a block of 16 (register j: element 2j + (tid & 1)) and end with its lower and upper
+// eight elements in order.  Half the values stay where they are, so four complex values a thread
+// cross by shuffles (an eighth of the data-pipe cycles of a shared-memory round trip) and
+// selects place them.  N = 2048 kernels: paired blind rotation 12.9 -> 11.7 us per bootstrap, 848
+// ragged bootstraps 4 % faster, no kernel slower.
+template <class C>
+__device__ __forceinline__ void tail_exchange_fwd(C (&x)[8], uint32_t tid) {
+    const bool b = tid & 1u;
+    C y[8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const C keep = b ? x[4 + r] : x[r], recv = shfl_pair(b ? x[r] : x[4 + r]);
+        y[2 * r] = b ? recv : keep;
+        y[2 * r + 1] = b ? keep : recv;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = y[j];
+}
+// its inverse
+template <class C>
+__device__ __forceinline__ void tail_exchange_inv(C (&x)[8], uint32_t tid) {
+    const bool b = tid & 1u;
+    C y[8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const C keep = b ? x[2 * r + 1] : x[2 * r], recv = shfl_pair(b ? x[2 * r] : x[2 * r + 1]);
+        y[r] = b ? recv : keep;
+        y[4 + r] = b ? keep : recv;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = y[j];
+}
+
 // Forward FFT of one folded polynomial by M/8 threads.  tab: the FftTab layout (in shared
 // memory); load(j, e) returns z_e = a_e + i a_(e+M) for register slot j (e < M); on return x[j] holds
 // spectrum slot 8*tid + j.  sm: M elements of shared memory, which the caller must not let
@@ -321,6 +362,11 @@ __device__ __forceinline__ void fft_forward_to_regs(C* sm, uint32_t tid, const C
     fwd_fft_pass<LOGM, 3>(x, 0, tid, tab);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
+        if (p == Pl::P - 1 && Pl::tail_r == 1) {
+            tail_exchange_fwd(x, tid);
+            fwd_fft_pass<LOGM, Pl::tail_r>(x, p, tid, tab);
+            break;
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[cswz_of<C>(pass_index<LOGM, 3>(1u << (3 * (p - 1)), tid, j))] = x[j];
         if (fwd_exchange_in_warp<LOGM>(p)) __syncwarp();
@@ -356,6 +402,13 @@ __device__ __forceinline__ void fft_forward2_to_regs(C* sm0, C* sm1, uint32_t ti
     fwd_fft_pass<LOGM, 3>(x1, 0, tid, tab);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
+        if (p == Pl::P - 1 && Pl::tail_r == 1) {
+            tail_exchange_fwd(x0, tid);
+            tail_exchange_fwd(x1, tid);
+            fwd_fft_pass<LOGM, Pl::tail_r>(x0, p, tid, tab);
+            fwd_fft_pass<LOGM, Pl::tail_r>(x1, p, tid, tab);
+            break;
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const uint32_t e = cswz_of<C>(pass_index<LOGM, 3>(1u << (3 * (p - 1)), tid, j));
@@ -398,15 +451,21 @@ __device__ __forceinline__ void fft_inverse_from_regs(C* sm, uint32_t tid, const
     using Pl = NttPlan<LOGM>;
     constexpr uint32_t mt = 1u << (3 * (Pl::P - 1));
     inv_fft_pass<LOGM, Pl::tail_r>(x, Pl::P - 1, tid, tab);
+    if (Pl::tail_r == 1) {
+        tail_exchange_inv(x, tid);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sm[cswz_of<C>(pass_index<LOGM, Pl::tail_r>(mt, tid, j))] = x[j];
-    if (inv_exchange_in_warp<LOGM>(Pl::P - 2)) __syncwarp();
-    else bar();
+        for (int j = 0; j < 8; ++j) sm[cswz_of<C>(pass_index<LOGM, Pl::tail_r>(mt, tid, j))] = x[j];
+        if (inv_exchange_in_warp<LOGM>(Pl::P - 2)) __syncwarp();
+        else bar();
+    }
 #pragma unroll
     for (int p = Pl::P - 2; p >= 0; --p) {
         const uint32_t m = 1u << (3 * p);
+        if (p < Pl::P - 2 || Pl::tail_r != 1) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = sm[cswz_of<C>(pass_index<LOGM, 3>(m, tid, j))];
+            for (int j = 0; j < 8; ++j) x[j] = sm[cswz_of<C>(pass_index<LOGM, 3>(m, tid, j))];
+        }
         inv_fft_pass<LOGM, 3>(x, p, tid, tab);
         if (p > 0) {
             // each pass reads and writes its own per-thread set and the sets partition [0, M), so
