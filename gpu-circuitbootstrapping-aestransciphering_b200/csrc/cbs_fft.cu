@@ -596,6 +596,8 @@ __global__ void __launch_bounds__(BrFftCfg<LOGN>::T, 1)
 // Measured at 296 ciphertexts (one wave, N = 2048, n = 630): 4.90 -> 3.83 ms (16.5 -> 12.9 us per
 // bootstrap) against spectra and outputs in shared memory, each thread forming one column from
 // three key loads at a time (62 % of the data-pipe cycles, the product phase waiting on L2).
+// With the transforms' tail exchange by shuffles 3.46 ms, with key batches two ahead (below)
+// 3.43 ms; 2368 ciphertexts: 11.5 us per bootstrap.
 template <int LOGN>
 __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
     k_blind_rotate_fft_mb2_x2(const BlindRotateArgs a, const FftKeyArgs f, uint32_t batch) {
@@ -726,34 +728,41 @@ __global__ void __launch_bounds__(4 * ((1u << LOGN) / 16), 1)
             at[c][0] = special_ms_f(__ldg(arow[c] + idx0), TWO_N, a.q_lwe, a.bitwidth);
             at[c][1] = idx1 < a.n ? special_ms_f(__ldg(arow[c] + idx1), TWO_N, a.q_lwe, a.bitwidth) : 0u;
         }
+        // 2. slots 2 pg, 2 pg + 1 of both columns of both ciphertexts.  Key batches (slot, row,
+        // column) of three subsets stream through registers, AHEAD batches loaded before the one in
+        // use, the first ones before the barrier.
+        const double2* gk = f.bskf + static_cast<size_t>(g) * KS * kstride + ht + 2 * pg * TH;
+        constexpr int BATCHES = 2 * L2 * 2, AHEAD = 2;
+        double2 kb[AHEAD + 1][KS];
+        auto load_keys = [&](int i) {
+            const double2* src = gk + (i / (2 * L2)) * TH + static_cast<size_t>(i % (2 * L2)) * M;
+#pragma unroll
+            for (uint32_t q = 0; q < KS; ++q) kb[i % (AHEAD + 1)][q] = __ldg(src + q * kstride);
+        };
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) load_keys(i);
         quad_sync();
-        // 2. slots 2 pg, 2 pg + 1 of both columns of both ciphertexts
-        const double2* gk = f.bskf + static_cast<size_t>(g) * KS * kstride + ht;
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj) {
             const uint32_t j = 2 * pg + jj;
-            const double2* kj = gk + j * TH;
             double2 s[2][2][KS];  // [column][ciphertext][subset]
 #pragma unroll
             for (uint32_t row = 0; row < L2; ++row) {  // row 2d + p: digit d of polynomial p
-                double2 k[2][KS];
-#pragma unroll
-                for (int col = 0; col < 2; ++col)
-#pragma unroll
-                    for (uint32_t q = 0; q < KS; ++q)
-                        k[col][q] = __ldg(kj + q * kstride + static_cast<size_t>(row * 2 + col) * M);
                 uint32_t xw[8];
                 tmem_load8(tspec + 32 * j + 8 * row, xw);
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const double2 x = tmem_complex(xw, c);
+                for (int col = 0; col < 2; ++col) {
+                    const int i = (jj * L2 + row) * 2 + col;
+                    if (i + AHEAD < BATCHES) load_keys(i + AHEAD);
 #pragma unroll
-                    for (int col = 0; col < 2; ++col)
+                    for (int c = 0; c < 2; ++c) {
+                        const double2 x = tmem_complex(xw, c);
 #pragma unroll
                         for (uint32_t q = 0; q < KS; ++q) {
-                            if (row == 0) s[col][c][q] = cmul(x, k[col][q]);
-                            else cfma(s[col][c][q], x, k[col][q]);
+                            if (row == 0) s[col][c][q] = cmul(x, kb[i % (AHEAD + 1)][q]);
+                            else cfma(s[col][c][q], x, kb[i % (AHEAD + 1)][q]);
                         }
+                    }
                 }
             }
 #pragma unroll
