@@ -1,0 +1,218 @@
+// br_solo.cuh -- grouped blind rotation (mb = 2) of one ciphertext by a whole CTA of 512 threads, or
+// by a cluster of two: the form for batches that leave SMs idle, where the time is the serial chain
+// of n/2 steps and not throughput.
+//
+// The throughput forms give a ciphertext 128 or 256 threads and let one SM work on several; a batch
+// below the SM count then runs at a quarter of an SM's warps, each step waiting on its own
+// transforms and key loads.  Here the 2 DIG digit transforms of a step run side by side, one per
+// M/8 threads, every thread forms one or two output slots with up to fifteen key loads in flight, and
+// the two inverse transforms follow: three barriers a step.  With two CTAs per ciphertext (CL = 2)
+// CTA r owns accumulator polynomial r, transforms its DIG digits, forms half of the slots from all
+// spectra (halves exchanged through distributed shared memory) and inverse-transforms output
+// column r, which halves the key bytes an SM has to pull per step, the floor of the one-CTA form
+// (its own L2 port: 64 bytes a cycle).
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "fft_core.cuh"
+#include "fft_ops.cuh"
+
+namespace cbs {
+
+template <int LOGN, int DIG, int CL>
+struct SoloCfg {
+    static constexpr int LOGM = LOGN - 1;
+    static constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, T = 512, W = T / TH;
+    static constexpr uint32_t POLYS = 2 / CL;              // accumulator polynomials of a CTA
+    static constexpr uint32_t ROWS = 2 * DIG / CL;         // digit transforms of a CTA
+    static constexpr uint32_t RECV = CL == 2 ? DIG * M / 2 : 0;  // the other CTA's spectra, this CTA's slots
+    static_assert(ROWS <= 2 * W, "at most two transforms per thread row");
+    using Tb = FftTab<LOGM>;
+    // shared memory in double2 units: tables, outputs [POLYS][M], spectra [ROWS][M], received
+    static constexpr uint32_t out_off = Tb::size(), row_off = out_off + POLYS * M, recv_off = row_off + ROWS * M,
+                              acc_off = recv_off + RECV;
+    static constexpr size_t smem(size_t word) { return acc_off * sizeof(double2) + POLYS * N * word; }
+};
+
+template <int CL>
+__device__ __forceinline__ uint32_t solo_rank() {
+    if constexpr (CL == 1) return 0;
+    else return blockIdx.x & 1u;  // cluster of two consecutive CTAs
+}
+template <int CL>
+__device__ __forceinline__ void solo_sync() {
+    if constexpr (CL == 1) __syncthreads();
+    else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// All groups of one ciphertext.  acc.digit(p, e, d): digit d of the folded pair at position e of the
+// CTA's polynomial p; acc.add(p, e, v): adds the inverse transform's pair v (untwisted, times M).
+// Both touch only positions e and e + M, and position e belongs to thread e mod M/8 of a row.
+// at(i): the rotation of LWE coefficient i (0 past n), the same in every thread.  keys: spectra
+// [groups][3 subsets][2 DIG][2][M] slot-major.  On return the accumulator is complete.
+template <int LOGN, int DIG, int CL, class Acc, class At>
+__device__ __forceinline__ void solo_groups(double2* sm, Acc& acc, const double2* __restrict__ keys, uint32_t groups,
+                                            At at) {
+    using Cfg = SoloCfg<LOGN, DIG, CL>;
+    constexpr int LOGM = Cfg::LOGM;
+    constexpr uint32_t M = Cfg::M, TH = Cfg::TH, W = Cfg::W, R = 2 * DIG, KS = 3;
+    constexpr size_t kstride = static_cast<size_t>(R) * 2 * M;
+    const uint32_t tid = threadIdx.x, wr = tid / TH, ht = tid % TH, rank = solo_rank<CL>();
+    const double2* tab = sm;
+    const double2* tws = tab + Cfg::Tb::twist_off();
+    double2* out = sm + Cfg::out_off;
+    double2* rows = sm + Cfg::row_off;
+    double2* recv = sm + Cfg::recv_off;
+    double2 *peer_out = nullptr, *peer_recv = nullptr;
+    if constexpr (CL == 2) {
+        auto cluster = cooperative_groups::this_cluster();
+        peer_out = cluster.map_shared_rank(out, rank ^ 1u);
+        peer_recv = cluster.map_shared_rank(recv, rank ^ 1u);
+    }
+    const uint32_t bar_id = 1 + wr;
+    auto row_bar = [bar_id]() { asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(TH) : "memory"); };
+    // row r of this CTA: digit d of its polynomial p
+    auto poly_of = [](uint32_t r) { return CL == 1 ? (r & 1u) : 0u; };
+    auto digit_of = [](uint32_t r) { return CL == 1 ? (r >> 1) : r; };
+    auto put = [&](uint32_t r, const double2 (&x)[8]) {
+        __syncwarp();
+        if constexpr (CL == 1) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) rows[r * M + cswz(8 * ht + j)] = x[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (static_cast<uint32_t>(j >> 2) == rank) rows[r * M + cswz(8 * ht + j)] = x[j];
+                else peer_recv[r * (M / 2) + (j & 3) * TH + ht] = x[j];
+            }
+        }
+    };
+    // product phase: slots (ht, j) of this thread, one or two columns
+    constexpr uint32_t SLOTS = M / CL;                            // of this CTA
+    constexpr int NS = SLOTS >= 512 ? SLOTS / 512 : 1, COLS = SLOTS >= 512 ? 2 : 1;
+    static_assert(SLOTS >= 256, "at least half a thread per slot");
+    const uint32_t j0 = CL == 1 ? wr : 4 * rank + (wr & 3u), col0 = COLS == 1 ? (wr >> 2) : 0u;
+    auto x_of = [&](uint32_t row, uint32_t j) {  // row 2d + p, slot (ht, j)
+        if constexpr (CL == 1) return rows[row * M + cswz(8 * ht + j)];
+        else
+            return (row & 1u) == rank ? rows[(row >> 1) * M + cswz(8 * ht + j)]
+                                      : recv[(row >> 1) * (M / 2) + (j & 3u) * TH + ht];
+    };
+    constexpr int BATCHES = NS * R * COLS, AHEAD = BATCHES < 4 ? BATCHES : 4;
+
+    for (uint32_t g = 0; g < groups; ++g) {
+        const uint32_t a0 = at(2 * g), a1 = at(2 * g + 1);
+        if ((a0 | a1) == 0) continue;  // every monomial factor is 0 (uniform over the cluster)
+        // 1. digit transforms, one per thread row (the first rows two where there are more)
+        if (wr + W < Cfg::ROWS) {
+            const uint32_t r0 = wr, r1 = wr + W;
+            double2 x0[8], x1[8];
+            fft_forward2_to_regs<LOGM>(
+                rows + r0 * M, rows + r1 * M, ht, tab,
+                [&](int, uint32_t e) { return acc.digit(poly_of(r0), e, digit_of(r0)); },
+                [&](int, uint32_t e) { return acc.digit(poly_of(r1), e, digit_of(r1)); }, x0, x1, row_bar);
+            put(r0, x0);
+            put(r1, x1);
+        } else if (wr < Cfg::ROWS) {
+            double2 x[8];
+            fft_forward_to_regs<LOGM>(
+                rows + wr * M, ht, tab, [&](int, uint32_t e) { return acc.digit(poly_of(wr), e, digit_of(wr)); }, x,
+                row_bar);
+            put(wr, x);
+        }
+        // 2. products: key batches (slot, row, column) of three subsets, AHEAD of them in flight
+        const double2* gk = keys + static_cast<size_t>(g) * KS * kstride + static_cast<size_t>(col0) * M + ht;
+        double2 kb[AHEAD + 1][KS];
+        auto load_keys = [&](int i) {
+            const int jj = i / (static_cast<int>(R) * COLS), rest = i % (static_cast<int>(R) * COLS);
+            const double2* src = gk + (j0 + W * jj) * TH + static_cast<size_t>(rest / COLS * 2 + rest % COLS) * M;
+#pragma unroll
+            for (uint32_t q = 0; q < KS; ++q) kb[i % (AHEAD + 1)][q] = __ldg(src + q * kstride);
+        };
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) load_keys(i);
+        solo_sync<CL>();
+#pragma unroll
+        for (int jj = 0; jj < NS; ++jj) {
+            const uint32_t j = j0 + W * jj;
+            double2 s[COLS][KS];
+#pragma unroll
+            for (uint32_t row = 0; row < R; ++row) {
+                const double2 x = x_of(row, j);
+#pragma unroll
+                for (int col = 0; col < COLS; ++col) {
+                    const int i = (jj * static_cast<int>(R) + static_cast<int>(row)) * COLS + col;
+                    if (i + AHEAD < BATCHES) load_keys(i + AHEAD);
+#pragma unroll
+                    for (uint32_t q = 0; q < KS; ++q) {
+                        if (row == 0) s[col][q] = cmul(x, kb[i % (AHEAD + 1)][q]);
+                        else cfma(s[col][q], x, kb[i % (AHEAD + 1)][q]);
+                    }
+                }
+            }
+            double2 c0 = zeta_pow<LOGN>(tws, slot_exp<LOGN>(mult_base<LOGN>(ht, a0), a0, j));
+            double2 c1 = zeta_pow<LOGN>(tws, slot_exp<LOGN>(mult_base<LOGN>(ht, a1), a1, j));
+            c0.x -= 1.0;
+            c1.x -= 1.0;
+#pragma unroll
+            for (int col = 0; col < COLS; ++col) {
+                // c0 (S_0 + c1 S_01) + c1 S_1
+                cfma(s[col][0], c1, s[col][2]);
+                double2 v = cmul(c0, s[col][0]);
+                cfma(v, c1, s[col][1]);
+                const uint32_t c = col0 + col, at_slot = j * TH + ht;
+                if constexpr (CL == 1) out[c * M + at_slot] = v;
+                else (c == rank ? out : peer_out)[at_slot] = v;
+            }
+        }
+        solo_sync<CL>();
+        // 3. inverse transforms of the CTA's columns
+        if (wr < Cfg::POLYS) {
+            double2 y[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[j] = out[wr * M + j * TH + ht];
+            fft_inverse_from_regs<LOGM>(
+                rows + wr * M, ht, tab, y,
+                [&](int j, uint32_t e, double2 v) { acc.add(wr, e, cmulc(v, twist_at<LOGM>(tws, j, e))); }, row_bar);
+        }
+        __syncthreads();
+    }
+}
+
+// launches of the solo kernels: opt-in shared memory and a cluster of CL CTAs
+template <int CL, class Kernel, class... Args>
+cudaError_t solo_launch(Kernel kernel, uint32_t ctas, size_t smem, cudaStream_t s, Args... args) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CL > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// CTAs per ciphertext for a batch on the current device: two while the clusters fit the SMs side by
+// side, one while the batch does, 0 above (the throughput forms)
+inline cudaError_t solo_ctas(uint32_t batch, uint32_t* out) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const uint32_t n = static_cast<uint32_t>(sms);
+    *out = 2 * batch <= n ? 2 : (batch <= n ? 1 : 0);
+    return cudaSuccess;
+}
+
+}  // namespace cbs

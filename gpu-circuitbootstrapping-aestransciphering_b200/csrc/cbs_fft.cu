@@ -970,8 +970,11 @@ cudaError_t launch_blind_rotate_fft_mb(const BlindRotateArgs& a, const FftKeyArg
     if (batch == 0) return cudaSuccess;
     if (mb < 2 || mb > 4) return cudaErrorInvalidValue;  // N = 4096: the per-slot c_i exceed shared memory
     if (a.g.gbits < 1 || a.g.gbits > 24 || a.digits < 1 || a.digits > 4) return cudaErrorInvalidValue;
-    cudaError_t e;
-    switch (N) {
+    cudaError_t e = cudaSuccess;
+    bool solo = false;
+    if (mb == 2 && a.by_batch) e = launch_blind_rotate_fft_solo(a, f, N, batch, s, &solo);
+    if (e != cudaSuccess) return e;
+    if (!solo) switch (N) {
         case 1024:
             e = mb == 2 ? br_fft_mb_launch<10, 2>(a, f, batch, s)
                         : (mb == 3 ? br_fft_mb_launch<10, 3>(a, f, batch, s) : br_fft_mb_launch<10, 4>(a, f, batch, s));

@@ -1,0 +1,98 @@
+// cbs_fft_solo.cu -- the CBS blind rotation (FP64 FFT, mb = 2) of a small batch, one ciphertext per
+// CTA or per cluster of two (br_solo.cuh); k_blind_rotate_fft_mb's arithmetic (offset-form
+// accumulator mod Q), finalize and multi-value split.
+//
+// Measured at N = 2048, n = 630, 2^18 x 2: 1-74 ciphertexts 1.98 ms (clusters of two), 75-148
+// 2.49 ms (one CTA each), against 2.90 ms lockstep and 3.40 ms paired; 149 up go to the paired form
+// (3.43 ms for 296, where two waves of this one would take 4.98).
+#include "common.cuh"
+#include "br_solo.cuh"
+#include "fft_kernels.cuh"
+
+namespace cbs {
+
+template <uint32_t M>
+struct CbsAcc {
+    int64_t* p;  // [polynomials][2 M], y = centre(x) + round_c in [lo, hi)
+    const FftKeyArgs& f;
+    int ign, gbits;
+    uint32_t fmask;
+    DigitBias bias;
+    int64_t lo, hi, Q;
+    __device__ __forceinline__ double2 digit(uint32_t poly, uint32_t e, uint32_t d) const {
+        return offset_digit_pair<M>(p + poly * 2 * M, e, ign + gbits * static_cast<int>(d), fmask, bias);
+    }
+    __device__ __forceinline__ void add(uint32_t poly, uint32_t e, double2 u) {
+        int64_t* y = p + poly * 2 * M;
+        y[e] = offset_add(y[e], centred_residue(u.x * f.inv_m, f), lo, hi, Q);
+        y[e + M] = offset_add(y[e + M], centred_residue(u.y * f.inv_m, f), lo, hi, Q);
+    }
+};
+
+template <int LOGN, int DIG, int CL>
+__global__ void __launch_bounds__(512, 1) k_blind_rotate_fft_solo(const BlindRotateArgs a, const FftKeyArgs f) {
+    using Cfg = SoloCfg<LOGN, DIG, CL>;
+    constexpr uint32_t N = Cfg::N, TWO_N = 2 * N;
+    extern __shared__ __align__(16) double2 solo_sm[];
+    const uint32_t tid = threadIdx.x, rank = solo_rank<CL>(), ct = blockIdx.x / CL;
+    const uint64_t Q = a.t.q, qhalf = Q >> 1;
+    const int gbits = a.g.gbits, ign = a.g.ign;
+    int64_t offset = 0;
+    for (int k = 0; k < DIG; ++k) offset += static_cast<int64_t>(1) << (gbits * k + gbits - 1);
+    const uint64_t round_c = (ign ? (uint64_t(1) << (ign - 1)) : 0) + (static_cast<uint64_t>(offset) << ign);
+    const int64_t hi = static_cast<int64_t>(round_c + qhalf), Qs = static_cast<int64_t>(Q), lo = hi - Qs;
+    auto to_offset = [&](uint64_t x) { return static_cast<int64_t>(x + round_c) - (x >= qhalf ? Qs : 0); };
+    for (uint32_t i = tid; i < Cfg::Tb::size(); i += Cfg::T) solo_sm[i] = f.tab[i];
+    int64_t* y = reinterpret_cast<int64_t*>(solo_sm + Cfg::acc_off);
+    const uint32_t bt = special_ms_f(a.b[ct], TWO_N, a.q_lwe, a.bitwidth);
+    for (uint32_t i = tid; i < Cfg::POLYS * N; i += Cfg::T) {
+        const uint32_t poly = CL == 1 ? i / N : rank, s = (i % N + bt) & (TWO_N - 1);
+        const uint64_t v = (s < N) ? a.tv[s] : a.tv[s - N];
+        y[i] = to_offset(poly == 0 ? 0 : ((s < N) ? v : (v ? Q - v : 0)));
+    }
+    CbsAcc<Cfg::M> acc{y, f, ign, gbits, (1u << gbits) - 1u, DigitBias(1u << (gbits - 1)), lo, hi, Qs};
+    const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
+    solo_sync<CL>();
+    solo_groups<LOGN, DIG, CL>(solo_sm, acc, f.bskf, (a.n + 1) / 2, [&](uint32_t i) {
+        return i < a.n ? special_ms_f(__ldg(arow + i), TWO_N, a.q_lwe, a.bitwidth) : 0u;
+    });
+    // finalize and the MV split, as in the one-bit form
+    uint64_t* x = reinterpret_cast<uint64_t*>(y);
+    for (uint32_t i = tid; i < Cfg::POLYS * N; i += Cfg::T) {
+        const uint32_t poly = CL == 1 ? i / N : rank, c = i % N;
+        const int64_t v0 = y[i] - static_cast<int64_t>(round_c);
+        uint64_t v = mul_shoup(static_cast<uint64_t>(v0 < 0 ? v0 + Qs : v0), a.t.n_inv, a.t.n_inv_s, Q);
+        if (poly == 1 && c < a.num_lut) v = add_mod(v, a.gadd[c], Q);
+        x[i] = v;
+    }
+    __syncthreads();
+    for (uint32_t j = 0; j < a.num_lut; ++j)
+        for (uint32_t i = tid; i < Cfg::POLYS * N; i += Cfg::T) {
+            const uint32_t poly = CL == 1 ? i / N : rank, s = i % N + j;
+            const uint64_t* src = x + (CL == 1 ? poly * N : 0);
+            a.mv_out[((static_cast<size_t>(ct) * a.num_lut + j) * 2 + poly) * N + i % N] =
+                (s < N) ? src[s] : (src[s - N] ? Q - src[s - N] : 0);
+        }
+}
+
+template <int LOGN, int DIG>
+static cudaError_t br_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch, uint32_t cl, cudaStream_t s) {
+    if (f.tab_len != FftTab<LOGN - 1>::size()) return cudaErrorInvalidValue;
+    if (cl == 2)
+        return solo_launch<2>(k_blind_rotate_fft_solo<LOGN, DIG, 2>, 2 * batch, SoloCfg<LOGN, DIG, 2>::smem(8), s, a, f);
+    return solo_launch<1>(k_blind_rotate_fft_solo<LOGN, DIG, 1>, batch, SoloCfg<LOGN, DIG, 1>::smem(8), s, a, f);
+}
+
+cudaError_t launch_blind_rotate_fft_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t batch,
+                                         cudaStream_t s, bool* taken) {
+    *taken = false;
+    if ((a.digits != 2 && a.digits != 3) || (N != 1024 && N != 2048)) return cudaSuccess;
+    uint32_t cl = 0;
+    cudaError_t e = solo_ctas(batch, &cl);
+    if (e != cudaSuccess || cl == 0) return e;
+    *taken = true;
+    if (N == 1024) return a.digits == 2 ? br_solo<10, 2>(a, f, batch, cl, s) : br_solo<10, 3>(a, f, batch, cl, s);
+    return a.digits == 2 ? br_solo<11, 2>(a, f, batch, cl, s) : br_solo<11, 3>(a, f, batch, cl, s);
+}
+
+}  // namespace cbs

@@ -38,6 +38,7 @@ struct BlindRotateArgs {
     const uint64_t* gadd;    // [num_lut] (gpow[j] >> 1) * N^-1 mod Q
     uint64_t* mv_out;        // [batch][num_lut][2][N] NTT domain (MV RLWEs after finalize)
     uint32_t schedule;       // FFT grouped form: CBS_BR_SCHEDULE_* (0 = the tuned / default choice)
+    bool by_batch;           // no schedule chosen by the caller: small batches take their own form
 };
 
 struct TraceArgs {

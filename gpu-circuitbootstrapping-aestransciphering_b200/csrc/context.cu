@@ -221,6 +221,7 @@ cbs_status run_blind_rotate(cbs_context* c, const uint64_t* d_a, const uint64_t*
     a.num_lut = c->p.num_lut;
     a.gadd = c->d_gadd.p;
     a.mv_out = d_mv;
+    a.by_batch = c->br_schedule == CBS_BR_SCHEDULE_AUTO;
     a.schedule = c->br_schedule != CBS_BR_SCHEDULE_AUTO ? c->br_schedule
                                                           : (c->has_tuned ? c->tuned.schedule : CBS_BR_SCHEDULE_AUTO);
     if (!mv_ntt && c->br_backend != CBS_BR_FFT64) {

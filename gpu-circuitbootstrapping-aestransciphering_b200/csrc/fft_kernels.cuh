@@ -100,6 +100,10 @@ cudaError_t launch_blind_rotate_fft(const BlindRotateArgs& a, const FftKeyArgs& 
 // [ceil(n/mb)][2^mb - 1][2*digits][2][N/2]
 cudaError_t launch_blind_rotate_fft_mb(const BlindRotateArgs& a, const FftKeyArgs& f, const cbs_dmodulus* d_mod,
                                        uint32_t N, uint32_t batch, uint32_t mb, cudaStream_t s, bool mv_ntt = true);
+// the small-batch form of mb = 2 (cbs_fft_solo.cu); *taken = false, nothing launched, where it does
+// not apply
+cudaError_t launch_blind_rotate_fft_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t batch,
+                                         cudaStream_t s, bool* taken);
 cudaError_t launch_trace_ss_fft(const TraceFftArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t count, cudaStream_t s);
 // digit spectra of the pair differences of `sets` fixed level-0 input sets (a.in, a.in_lut_stride,
 // a.in_count, a.g, a.digits) into out [sets][in_count/2][2*digits][N/2]

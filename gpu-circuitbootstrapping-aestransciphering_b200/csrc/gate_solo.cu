@@ -1,0 +1,88 @@
+// gate_solo.cu -- the torus blind rotation (gates, torus circuit bootstrap) of a small batch, one
+// ciphertext per CTA or per cluster of two (br_solo.cuh); the products round to the same integers as
+// k_gate_blind_rotate_mb's, so the 32-bit results are the same words.
+//
+// Measured, grouped mb = 2: 64 gates (n = 636, N = 1024; clusters of two) 2.88 -> 1.51 ms, 144
+// level-2 rotations (n = 630, N = 2048, 64-bit torus; one CTA each) 3.85 -> 3.3 ms.
+#include "common.cuh"
+#include "br_solo.cuh"
+#include "gate_ops.cuh"
+
+namespace cbs {
+
+template <typename TT, uint32_t M>
+struct TorusAcc {
+    TT* p;  // [polynomials][2 M]
+    TT off;
+    uint32_t bg, fmask;
+    DigitBias bias;
+    __device__ __forceinline__ double2 digit(uint32_t poly, uint32_t e, uint32_t d) const {
+        const TT* a = p + poly * 2 * M;
+        const uint32_t sft = 8 * sizeof(TT) - (d + 1) * bg;
+        return make_double2(bias(static_cast<uint32_t>((a[e] + off) >> sft) & fmask),
+                            bias(static_cast<uint32_t>((a[e + M] + off) >> sft) & fmask));
+    }
+    __device__ __forceinline__ void add(uint32_t poly, uint32_t e, double2 u) {
+        constexpr double inv_m = 1.0 / M;
+        TT* a = p + poly * 2 * M;
+        a[e] += to_torus<TT>(u.x * inv_m);
+        a[e + M] += to_torus<TT>(u.y * inv_m);
+    }
+};
+
+template <int LOGN, int DIG, int CL, typename TT>
+__global__ void __launch_bounds__(512, 1) k_gate_solo(const GateArgs a) {
+    using Cfg = SoloCfg<LOGN, DIG, CL>;
+    constexpr uint32_t N = Cfg::N, TWO_N = 2 * N, SH = 32 - (LOGN + 1), W = 8 * sizeof(TT);
+    extern __shared__ __align__(16) double2 solo_sm[];
+    const uint32_t tid = threadIdx.x, rank = solo_rank<CL>(), item = blockIdx.x / CL;
+    for (uint32_t i = tid; i < Cfg::Tb::size(); i += Cfg::T) solo_sm[i] = a.tab[i];
+    auto ms = [](uint32_t x) { return ((x + (1u << (SH - 1))) >> SH) & (TWO_N - 1); };
+    const uint32_t *a1, *a2;
+    uint32_t b;
+    gate_item_inputs(a, item, a1, a2, b);
+    const TT mu = static_cast<TT>(a.mu[item % a.levels_tv]), b_add = static_cast<TT>(a.b_add[item % a.levels_tv]);
+    TT* accp = reinterpret_cast<TT*>(solo_sm + Cfg::acc_off);
+    TT off = TT(1) << (W - DIG * a.bg_bits - 1);
+    for (uint32_t k = 0; k < DIG; ++k) off += (TT(1) << (a.bg_bits - 1)) << (W - (k + 1) * a.bg_bits);
+    const uint32_t bt = ms(b);
+    for (uint32_t i = tid; i < Cfg::POLYS * N; i += Cfg::T) {
+        const uint32_t poly = CL == 1 ? i / N : rank, c = i % N;
+        const uint32_t sp = (c + bt) & (TWO_N - 1);
+        const TT tv = a.tv ? static_cast<TT>(__ldg(a.tv + (sp & (N - 1)))) : mu;
+        accp[i] = poly == 0 ? TT(0) : (sp < N ? tv : TT(0) - tv);
+    }
+    TorusAcc<TT, Cfg::M> acc{accp, off, a.bg_bits, (1u << a.bg_bits) - 1u, DigitBias(1u << (a.bg_bits - 1))};
+    solo_sync<CL>();
+    solo_groups<LOGN, DIG, CL>(solo_sm, acc, a.bskf, (a.n + 1) / 2, [&](uint32_t i) {
+        return i < a.n ? ms(a.reqs ? __ldg(a1 + i) : gate_a(a.gate, __ldg(a1 + i), __ldg(a2 + i))) : 0u;
+    });
+    // sample extract of coefficient 0: a'_0 = a_0, a'_i = -a_(N-i), b' = b_0
+    TT* out = reinterpret_cast<TT*>(a.ext) + static_cast<size_t>(item) * (N + 1);
+    if (rank == 0)
+        for (uint32_t i = tid; i < N; i += Cfg::T) out[i] = i == 0 ? accp[0] : TT(0) - accp[N - i];
+    if (tid == 0 && (CL == 1 || rank == 1)) out[N] = accp[CL == 1 ? N : 0] + b_add;
+}
+
+template <int LOGN, int DIG, typename TT>
+static cudaError_t gate_solo(const GateArgs& a, uint32_t cl, cudaStream_t s) {
+    if (cl == 2)
+        return solo_launch<2>(k_gate_solo<LOGN, DIG, 2, TT>, 2 * a.items, SoloCfg<LOGN, DIG, 2>::smem(sizeof(TT)), s, a);
+    return solo_launch<1>(k_gate_solo<LOGN, DIG, 1, TT>, a.items, SoloCfg<LOGN, DIG, 1>::smem(sizeof(TT)), s, a);
+}
+
+template <typename TT>
+cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s, bool* taken) {
+    *taken = false;
+    if (a.mb != 2 || a.fft_mode != 0 || (a.levels != 2 && a.levels != 3) || (N != 1024 && N != 2048)) return cudaSuccess;
+    uint32_t cl = 0;
+    cudaError_t e = solo_ctas(a.items, &cl);
+    if (e != cudaSuccess || cl == 0) return e;
+    *taken = true;
+    if (N == 1024) return a.levels == 2 ? gate_solo<10, 2, TT>(a, cl, s) : gate_solo<10, 3, TT>(a, cl, s);
+    return a.levels == 2 ? gate_solo<11, 2, TT>(a, cl, s) : gate_solo<11, 3, TT>(a, cl, s);
+}
+template cudaError_t gate_blind_rotate_solo<uint32_t>(const GateArgs&, uint32_t, cudaStream_t, bool*);
+template cudaError_t gate_blind_rotate_solo<uint64_t>(const GateArgs&, uint32_t, cudaStream_t, bool*);
+
+}  // namespace cbs

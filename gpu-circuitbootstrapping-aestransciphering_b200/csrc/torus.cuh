@@ -56,6 +56,9 @@ struct GateArgs {
 
 cudaError_t gate_blind_rotate(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);    // 32-bit torus
 cudaError_t gate_blind_rotate64(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);  // 64-bit torus
+// the small-batch form (gate_solo.cu); *taken = false, nothing launched, where it does not apply
+template <typename TT>
+cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s, bool* taken);
 
 uint32_t torus_from_double(double x);
 uint32_t torus_noise(Rng& rng, double sigma);
