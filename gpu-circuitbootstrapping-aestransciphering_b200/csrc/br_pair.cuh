@@ -1,0 +1,315 @@
+// br_pair.cuh -- grouped blind rotation (mb = 2) of two ciphertexts per lane set, the throughput
+// form: 512 threads per CTA, 16 warps per SM, every key word loaded feeds two ciphertexts.
+//
+// Thread ht of each M/8-thread row (ciphertext, polynomial) transforms the digits of its polynomial
+// (two in lockstep, a third after them) and ends with slots 8 ht .. 8 ht + 7; everything that
+// passes between the phases of a step stays in its lane, so it goes through tensor memory (TMEM)
+// and not through shared memory, which the transforms' exchanges keep busy:
+//  * the accumulator: the transform reads and writes the same 16 coefficients every step (positions
+//    e, e + M of its 8 slots);
+//  * the digit spectra, per slot [row][ciphertext];
+//  * the outputs, in columns of their own where they are left, else in the place of spectrum row
+//    `column` of the same slot and ciphertext, which the row that reads the output writes next.
+// A warp reaches the lanes of its TMEM quadrant only, which are the same lanes in the four rows: the
+// four warps of a quadrant exchange spectra and outputs among themselves, so the two barriers around
+// the product phase join 128 threads, not the CTA.  At N = 2048 a row covers the 128 lanes (one lane
+// set, two ciphertexts per CTA), at N = 1024 64 of them (two sets, four ciphertexts).
+// Per step: 1. digit transforms, spectra to TMEM; 2. row pg of a lane forms slots 2 pg and 2 pg + 1 of
+// both output columns of both ciphertexts: per column and subset S the sums sum_row x_row K_S[row]
+// (key batches two ahead: the phase is bound by the latency and the rate of these loads), then
+// c_0 (S_0 + c_1 S_01) + c_1 S_1 with c_i(psi) = psi^(a_i) - 1; 3. each row inverse-transforms its
+// column and adds the rounded result into its accumulator.
+//
+// Measured on 592 torus bootstraps (three levels, one wave at N = 1024 / two at N = 2048): 6.63 ->
+// 4.49 ms and 15.02 -> 9.08 ms against k_gate_blind_rotate_mb; with the rotations switched from the
+// inputs every step instead of once into shared memory 5.12 and 11.53 ms.
+#pragma once
+
+#include "fft_core.cuh"
+#include "fft_ops.cuh"
+#include "tmem.cuh"
+
+namespace cbs {
+
+// WORDS: 32-bit words of an accumulator coefficient
+template <int LOGN, int DIG, int WORDS>
+struct PairCfg {
+    static constexpr int LOGM = LOGN - 1;
+    static constexpr uint32_t N = 1u << LOGN, M = N / 2, TH = M / 8, T = 512, SETS = 128 / TH;
+    static_assert(TH == 64 || TH == 128, "a lane set is 64 or 128 lanes");
+    static constexpr uint32_t CTS = 2 * SETS;                       // ciphertexts per CTA
+    static constexpr uint32_t ACC_COLS = 16 * WORDS, SLOT_COLS = 16 * DIG, SPEC_COL = 4 * ACC_COLS;
+    static_assert(SPEC_COL + 8 * SLOT_COLS <= 512, "TMEM columns");
+    // outputs in columns of their own (32 per row, one load) where they are left
+    static constexpr bool OWN_OUT = SPEC_COL + 8 * SLOT_COLS + 128 <= 512;
+    static constexpr uint32_t OUT_COL = SPEC_COL + 8 * SLOT_COLS;
+    using Tb = FftTab<LOGM>;
+    // shared memory: tables, TMEM address, then [4 rows][SETS] exchange buffers of 2 M
+    static constexpr size_t slot_off = (Tb::size() * sizeof(double2) + 15) / 16 * 16, buf_off = slot_off + 16;
+    static constexpr size_t rot_off = buf_off + 4ull * SETS * 2 * M * sizeof(double2);
+    // and the rotations of every LWE coefficient, [CTS][2 groups] 16-bit
+    static constexpr size_t smem(uint32_t n) { return rot_off + CTS * rot_stride(n) * sizeof(uint16_t); }
+    static constexpr uint32_t rot_stride(uint32_t n) { return (n + 1) & ~1u; }
+};
+
+// a thread's place: row (c2, h) = (ciphertext of the set, polynomial), lane l = 32 (warp mod 4) + lane
+template <int LOGN, int DIG, int WORDS>
+struct PairThread {
+    using Cfg = PairCfg<LOGN, DIG, WORDS>;
+    uint32_t row, c2, h, set, ht;
+    double2 *tab, *buf;
+    uint16_t* rot;  // of the set's two ciphertexts, n padded to even
+    uint32_t tmem;
+    __device__ __forceinline__ PairThread(uint8_t* smem, uint32_t n) {
+        const uint32_t l = threadIdx.x % 128;
+        row = threadIdx.x / 128, c2 = row >> 1, h = row & 1u, set = l / Cfg::TH, ht = l % Cfg::TH;
+        tab = reinterpret_cast<double2*>(smem);
+        buf = reinterpret_cast<double2*>(smem + Cfg::buf_off) + (row * Cfg::SETS + set) * 2 * Cfg::M;
+        rot = reinterpret_cast<uint16_t*>(smem + Cfg::rot_off) + 2 * set * Cfg::rot_stride(n);
+        tmem = 0;
+    }
+    __device__ __forceinline__ uint32_t acc_addr() const { return tmem_quadrant_addr(tmem, row * Cfg::ACC_COLS); }
+};
+
+// tables and TMEM (512 columns: the CTA's shared memory keeps a second one off the SM)
+template <class Th>
+__device__ __forceinline__ void pair_begin(Th& th, uint8_t* smem, const double2* table) {
+    using Cfg = typename Th::Cfg;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(smem + Cfg::slot_off);
+    if (threadIdx.x < 32) tmem_alloc(slot, 512);
+    for (uint32_t i = threadIdx.x; i < Cfg::Tb::size(); i += Cfg::T) th.tab[i] = table[i];
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    th.tmem = *slot;
+}
+template <class Th>
+__device__ __forceinline__ void pair_end(const Th& th) {
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    if (threadIdx.x < 32) tmem_dealloc(th.tmem, 512);
+}
+
+// the rotations of the set's ciphertexts (row c2's ciphertext by its 2 TH threads): of(i) in [0, 2 N)
+template <class Th, class Of>
+__device__ __forceinline__ void pair_rotations(const Th& th, uint32_t n, Of of) {
+    using Cfg = typename Th::Cfg;
+    uint16_t* r = th.rot + th.c2 * Cfg::rot_stride(n);
+    for (uint32_t i = th.h * Cfg::TH + th.ht; i < Cfg::rot_stride(n); i += 2 * Cfg::TH)
+        r[i] = static_cast<uint16_t>(i < n ? of(i) : 0u);
+}
+
+// accumulator coefficient q (of 16: 2 j = position e_j, 2 j + 1 = e_j + M) within a thread's words
+template <class Word>
+__device__ __forceinline__ Word pair_get(const uint32_t (&w)[16], int q) {
+    if constexpr (sizeof(Word) == 4) return static_cast<Word>(w[q]);
+    else return static_cast<Word>(static_cast<uint64_t>(w[2 * q]) | (static_cast<uint64_t>(w[2 * q + 1]) << 32));
+}
+template <class Word>
+__device__ __forceinline__ void pair_set(uint32_t (&w)[16], int q, Word v) {
+    if constexpr (sizeof(Word) == 4) w[q] = static_cast<uint32_t>(v);
+    else {
+        w[2 * q] = static_cast<uint32_t>(static_cast<uint64_t>(v));
+        w[2 * q + 1] = static_cast<uint32_t>(static_cast<uint64_t>(v) >> 32);
+    }
+}
+// blocks of 16 columns hold HALF slots (8 for 32-bit words, 4 for 64-bit words)
+template <class Word>
+constexpr int pair_half() { return sizeof(Word) == 4 ? 8 : 4; }
+
+// the thread's accumulator words from init(e) (position e of polynomial h; e < 2 M)
+template <class Word, class Th, class Init>
+__device__ __forceinline__ void pair_init(const Th& th, Init init) {
+    using Cfg = typename Th::Cfg;
+    constexpr int HALF = pair_half<Word>();
+#pragma unroll
+    for (int b = 0; b < 8 / HALF; ++b) {
+        uint32_t w[16];
+#pragma unroll
+        for (int jj = 0; jj < HALF; ++jj) {
+            const uint32_t e = pass_index<Cfg::LOGM, 3>(1u, th.ht, HALF * b + jj);
+            pair_set<Word>(w, 2 * jj, init(e));
+            pair_set<Word>(w, 2 * jj + 1, init(e + Cfg::M));
+        }
+        tmem_store16(th.acc_addr() + 16 * b, w);
+    }
+    tmem_wait_store();
+}
+// and out: give(e, word)
+template <class Word, class Th, class Give>
+__device__ __forceinline__ void pair_read(const Th& th, Give give) {
+    using Cfg = typename Th::Cfg;
+    constexpr int HALF = pair_half<Word>();
+#pragma unroll
+    for (int b = 0; b < 8 / HALF; ++b) {
+        uint32_t w[16];
+        tmem_load16(th.acc_addr() + 16 * b, w);
+#pragma unroll
+        for (int jj = 0; jj < HALF; ++jj) {
+            const uint32_t e = pass_index<Cfg::LOGM, 3>(1u, th.ht, HALF * b + jj);
+            give(e, pair_get<Word>(w, 2 * jj));
+            give(e + Cfg::M, pair_get<Word>(w, 2 * jj + 1));
+        }
+    }
+}
+
+// All groups of the CTA's ciphertexts.  Acc: Word, digit(word, d) (FP64), add(word, v) with v an
+// untwisted output of the inverse transform, times M.  n: LWE coefficients (pair_rotations before a
+// CTA barrier).  keys: spectra [groups][3 subsets][2 DIG][2][M] slot-major.
+template <int LOGN, int DIG, class Acc, class Th>
+__device__ __forceinline__ void pair_groups(const Th& th, const Acc& acc, const double2* __restrict__ keys,
+                                            uint32_t n) {
+    using Cfg = typename Th::Cfg;
+    using Word = typename Acc::Word;
+    constexpr int LOGM = Cfg::LOGM, HALF = pair_half<Word>();
+    constexpr uint32_t M = Cfg::M, TH = Cfg::TH, R = 2 * DIG, KS = 3;
+    constexpr size_t kstride = static_cast<size_t>(R) * 2 * M;  // spectra between subsets of a group
+    const double2* tab = th.tab;
+    const double2* tws = tab + Cfg::Tb::twist_off();
+    double2 *buf0 = th.buf, *buf1 = th.buf + M;
+    const uint32_t ht = th.ht, c2 = th.c2, h = th.h, pg = th.row;
+    const uint32_t tacc = th.acc_addr(), tspec = tmem_quadrant_addr(th.tmem, Cfg::SPEC_COL);
+    // named barriers: one per row of a lane set, one per lane quadrant
+    const uint32_t row_id = 1 + th.row * Cfg::SETS + th.set, quad_id = 9 + (threadIdx.x % 128) / 32;
+    auto row_bar = [row_id]() { asm volatile("bar.sync %0, %1;" ::"r"(row_id), "n"(TH) : "memory"); };
+    auto quad_sync = [quad_id]() {  // this thread's TMEM stores are visible to the quadrant's warps after it
+        tmem_wait_store();
+        tmem_fence_before();
+        asm volatile("bar.sync %0, %1;" ::"r"(quad_id), "n"(128) : "memory");
+        tmem_fence_after();
+    };
+    [[maybe_unused]] const uint32_t tout = tmem_quadrant_addr(th.tmem, Cfg::OUT_COL);
+    auto place = [&](int j, uint32_t row, uint32_t c) {
+        return tspec + static_cast<uint32_t>(j) * Cfg::SLOT_COLS + 8 * row + 4 * c;
+    };
+    const uint32_t groups = (n + 1) / 2;
+    for (uint32_t g = 0; g < groups; ++g) {
+        // 1. digit transforms of polynomial h, digits read from the accumulator; rows 2 d + h
+        {
+            uint32_t w[8 / HALF][16];
+#pragma unroll
+            for (int b = 0; b < 8 / HALF; ++b) tmem_load16(tacc + 16 * b, w[b]);
+            auto pair_of = [&](int j, int d) {
+                const uint32_t(&v)[16] = w[j / HALF];
+                return make_double2(acc.digit(pair_get<Word>(v, 2 * (j % HALF)), d),
+                                    acc.digit(pair_get<Word>(v, 2 * (j % HALF) + 1), d));
+            };
+            double2 x0[8], x1[8];
+            fft_forward2_to_regs<LOGM>(
+                buf0, buf1, ht, tab, [&](int j, uint32_t) { return pair_of(j, 0); },
+                [&](int j, uint32_t) { return pair_of(j, 1); }, x0, x1, row_bar);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                tmem_store_complex(place(j, h, c2), x0[j]);
+                tmem_store_complex(place(j, 2 + h, c2), x1[j]);
+            }
+            if constexpr (DIG == 3) {
+                row_bar();  // the lockstep pair's reads of buf0 are done
+                uint32_t w2[8 / HALF][16];
+#pragma unroll
+                for (int b = 0; b < 8 / HALF; ++b) tmem_load16(tacc + 16 * b, w2[b]);
+                fft_forward_to_regs<LOGM>(
+                    buf0, ht, tab,
+                    [&](int j, uint32_t) {
+                        const uint32_t(&v)[16] = w2[j / HALF];
+                        return make_double2(acc.digit(pair_get<Word>(v, 2 * (j % HALF)), 2),
+                                            acc.digit(pair_get<Word>(v, 2 * (j % HALF) + 1), 2));
+                    },
+                    x0, row_bar);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) tmem_store_complex(place(j, 4 + h, c2), x0[j]);
+            }
+        }
+        // 2. slots 2 pg, 2 pg + 1 of both columns of both ciphertexts.  Key batches (slot, row,
+        // column) of three subsets stream through registers, AHEAD batches loaded before the one in
+        // use, the first ones before the barrier.
+        const double2* gk = keys + static_cast<size_t>(g) * KS * kstride + ht + 2 * pg * TH;
+        constexpr int BATCHES = 2 * R * 2, AHEAD = 2;
+        double2 kb[AHEAD + 1][KS];
+        auto load_keys = [&](int i) {
+            const double2* src = gk + (i / (2 * static_cast<int>(R))) * TH +
+                                 static_cast<size_t>(i % (2 * static_cast<int>(R))) * M;
+#pragma unroll
+            for (uint32_t q = 0; q < KS; ++q) kb[i % (AHEAD + 1)][q] = __ldg(src + q * kstride);
+        };
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) load_keys(i);
+        quad_sync();
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+            const uint32_t j = 2 * pg + jj;
+            double2 s[2][2][KS];  // [column][ciphertext][subset]
+#pragma unroll
+            for (uint32_t row = 0; row < R; ++row) {  // row 2d + p: digit d of polynomial p
+                uint32_t xw[8];
+                tmem_load8(place(static_cast<int>(j), row, 0), xw);
+#pragma unroll
+                for (int col = 0; col < 2; ++col) {
+                    const int i = (jj * static_cast<int>(R) + static_cast<int>(row)) * 2 + col;
+                    if (i + AHEAD < BATCHES) load_keys(i + AHEAD);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const double2 x = tmem_complex(xw, c);
+#pragma unroll
+                        for (uint32_t q = 0; q < KS; ++q) {
+                            if (row == 0) s[col][c][q] = cmul(x, kb[i % (AHEAD + 1)][q]);
+                            else cfma(s[col][c][q], x, kb[i % (AHEAD + 1)][q]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                double2 cc[2];  // c_i(psi) of this slot
+                const uint32_t both = *reinterpret_cast<const uint32_t*>(th.rot + c * Cfg::rot_stride(n) + 2 * g);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t r = i ? both >> 16 : both & 0xffffu;
+                    cc[i] = zeta_pow<LOGN>(tws, slot_exp<LOGN>(mult_base<LOGN>(ht, r), r, j));
+                    cc[i].x -= 1.0;
+                }
+#pragma unroll
+                for (int col = 0; col < 2; ++col) {
+                    cfma(s[col][c][0], cc[1], s[col][c][2]);
+                    double2 v = cmul(cc[0], s[col][c][0]);
+                    cfma(v, cc[1], s[col][c][1]);
+                    if constexpr (Cfg::OWN_OUT) tmem_store_complex(tout + 32 * (2 * c + col) + 4 * j, v);
+                    else tmem_store_complex(place(static_cast<int>(j), col, c), v);
+                }
+            }
+        }
+        quad_sync();
+        double2 yv[8];
+        if constexpr (Cfg::OWN_OUT) {
+            uint32_t w[32];
+            tmem_load32(tout + 32 * th.row, w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) yv[j] = tmem_complex(w, j);
+        } else {
+            uint32_t w[8][4];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) tmem_load4_nowait(place(j, h, c2), w[j]);
+            tmem_wait_load(w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) yv[j] = tmem_complex(w[j], 0);
+        }
+        // 3. inverse transform, rounding, accumulate (each 16-column block read when its first slot
+        // arrives, written back after its last)
+        uint32_t wacc[16];
+        fft_inverse_from_regs<LOGM>(
+            buf0, ht, tab, yv,
+            [&](int j, uint32_t e, double2 v) {
+                const int jj = j % HALF;
+                if (jj == 0) tmem_load16(tacc + 16 * (j / HALF), wacc);
+                const double2 u = cmulc(v, twist_at<LOGM>(tws, j, e));
+                pair_set<Word>(wacc, 2 * jj, acc.add(pair_get<Word>(wacc, 2 * jj), u.x));
+                pair_set<Word>(wacc, 2 * jj + 1, acc.add(pair_get<Word>(wacc, 2 * jj + 1), u.y));
+                if (jj == HALF - 1) tmem_store16(tacc + 16 * (j / HALF), wacc);
+            },
+            row_bar);
+        tmem_wait_store();
+    }
+}
+
+}  // namespace cbs

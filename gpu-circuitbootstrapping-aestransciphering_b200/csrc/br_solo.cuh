@@ -32,7 +32,9 @@ struct SoloCfg {
     // shared memory in double2 units: tables, outputs [POLYS][M], spectra [ROWS][M], received
     static constexpr uint32_t out_off = Tb::size(), row_off = out_off + POLYS * M, recv_off = row_off + ROWS * M,
                               acc_off = recv_off + RECV;
-    static constexpr size_t smem(size_t word) { return acc_off * sizeof(double2) + POLYS * N * word; }
+    // accumulator words [POLYS][N], then the rotations of every LWE coefficient (16-bit, n even)
+    static constexpr size_t rot_off(size_t word) { return acc_off * sizeof(double2) + POLYS * N * word; }
+    static constexpr size_t smem(size_t word, uint32_t n) { return rot_off(word) + ((n + 1) & ~1u) * sizeof(uint16_t); }
 };
 
 template <int CL>
@@ -52,11 +54,11 @@ __device__ __forceinline__ void solo_sync() {
 // All groups of one ciphertext.  acc.digit(p, e, d): digit d of the folded pair at position e of the
 // CTA's polynomial p; acc.add(p, e, v): adds the inverse transform's pair v (untwisted, times M).
 // Both touch only positions e and e + M, and position e belongs to thread e mod M/8 of a row.
-// at(i): the rotation of LWE coefficient i (0 past n), the same in every thread.  keys: spectra
-// [groups][3 subsets][2 DIG][2][M] slot-major.  On return the accumulator is complete.
-template <int LOGN, int DIG, int CL, class Acc, class At>
+// rot: the rotations in [0, 2 N) of the 2 groups LWE coefficients (0 past n), in shared memory.
+// keys: spectra [groups][3 subsets][2 DIG][2][M] slot-major.  On return the accumulator is complete.
+template <int LOGN, int DIG, int CL, class Acc>
 __device__ __forceinline__ void solo_groups(double2* sm, Acc& acc, const double2* __restrict__ keys, uint32_t groups,
-                                            At at) {
+                                            const uint16_t* rot) {
     using Cfg = SoloCfg<LOGN, DIG, CL>;
     constexpr int LOGM = Cfg::LOGM;
     constexpr uint32_t M = Cfg::M, TH = Cfg::TH, W = Cfg::W, R = 2 * DIG, KS = 3;
@@ -105,7 +107,7 @@ __device__ __forceinline__ void solo_groups(double2* sm, Acc& acc, const double2
     constexpr int BATCHES = NS * R * COLS, AHEAD = BATCHES < 4 ? BATCHES : 4;
 
     for (uint32_t g = 0; g < groups; ++g) {
-        const uint32_t a0 = at(2 * g), a1 = at(2 * g + 1);
+        const uint32_t both = *reinterpret_cast<const uint32_t*>(rot + 2 * g), a0 = both & 0xffffu, a1 = both >> 16;
         if ((a0 | a1) == 0) continue;  // every monomial factor is 0 (uniform over the cluster)
         // 1. digit transforms, one per thread row (the first rows two where there are more)
         if (wr + W < Cfg::ROWS) {
@@ -183,6 +185,15 @@ __device__ __forceinline__ void solo_groups(double2* sm, Acc& acc, const double2
     }
 }
 
+// CTAs per ciphertext: two while the clusters fit the SMs side by side
+inline cudaError_t solo_ctas(uint32_t batch, uint32_t* out) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    *out = 2 * static_cast<uint64_t>(batch) <= static_cast<uint64_t>(sms) ? 2 : 1;
+    return e;
+}
+
 // launches of the solo kernels: opt-in shared memory and a cluster of CL CTAs
 template <int CL, class Kernel, class... Args>
 cudaError_t solo_launch(Kernel kernel, uint32_t ctas, size_t smem, cudaStream_t s, Args... args) {
@@ -201,18 +212,6 @@ cudaError_t solo_launch(Kernel kernel, uint32_t ctas, size_t smem, cudaStream_t 
     cfg.attrs = attr;
     cfg.numAttrs = CL > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-// CTAs per ciphertext for a batch on the current device: two while the clusters fit the SMs side by
-// side, one while the batch does, 0 above (the throughput forms)
-inline cudaError_t solo_ctas(uint32_t batch, uint32_t* out) {
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    const uint32_t n = static_cast<uint32_t>(sms);
-    *out = 2 * batch <= n ? 2 : (batch <= n ? 1 : 0);
-    return cudaSuccess;
 }
 
 }  // namespace cbs

@@ -953,8 +953,10 @@ static cudaError_t br_fft_mb_launch(const BlindRotateArgs& a, const FftKeyArgs& 
     if constexpr (MB == 2 && LOGN == 11) {
         // two ciphertexts per CTA (digits read from the accumulator: any digit width up to 24
         // bits); also the default when no schedule was chosen or tuned (the fastest form on B200)
-        if (a.digits == 2 && (a.schedule == CBS_BR_SCHEDULE_PAIRED || a.schedule == CBS_BR_SCHEDULE_AUTO))
-            return br_fft_mb2_x2_launch<LOGN>(a, f, batch, s);
+        if ((a.digits == 2 || a.digits == 3) &&
+            (a.schedule == CBS_BR_SCHEDULE_PAIRED || a.schedule == CBS_BR_SCHEDULE_AUTO))
+            return a.digits == 2 ? br_fft_mb2_x2_launch<LOGN>(a, f, batch, s)
+                                 : launch_blind_rotate_fft_pair3(a, f, batch, s);
     }
     if constexpr (MB == 2) {
         // the two-digit gadget: both digit transforms in lockstep unless the digit-by-digit
@@ -971,19 +973,28 @@ cudaError_t launch_blind_rotate_fft_mb(const BlindRotateArgs& a, const FftKeyArg
     if (mb < 2 || mb > 4) return cudaErrorInvalidValue;  // N = 4096: the per-slot c_i exceed shared memory
     if (a.g.gbits < 1 || a.g.gbits > 24 || a.digits < 1 || a.digits > 4) return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
-    bool solo = false;
-    if (mb == 2 && a.by_batch) e = launch_blind_rotate_fft_solo(a, f, N, batch, s, &solo);
+    // what a wave leaves over takes the small-batch form (solo_rest has the rule)
+    uint32_t rest = 0;
+    if (mb == 2 && a.by_batch && (a.digits == 2 || a.digits == 3)) e = solo_rest(batch, N == 2048 ? 2 : 0, &rest);
     if (e != cudaSuccess) return e;
-    if (!solo) switch (N) {
+    const uint32_t most = batch - rest;
+    if (most) switch (N) {
         case 1024:
-            e = mb == 2 ? br_fft_mb_launch<10, 2>(a, f, batch, s)
-                        : (mb == 3 ? br_fft_mb_launch<10, 3>(a, f, batch, s) : br_fft_mb_launch<10, 4>(a, f, batch, s));
+            e = mb == 2 ? br_fft_mb_launch<10, 2>(a, f, most, s)
+                        : (mb == 3 ? br_fft_mb_launch<10, 3>(a, f, most, s) : br_fft_mb_launch<10, 4>(a, f, most, s));
             break;
         case 2048:
-            e = mb == 2 ? br_fft_mb_launch<11, 2>(a, f, batch, s)
-                        : (mb == 3 ? br_fft_mb_launch<11, 3>(a, f, batch, s) : br_fft_mb_launch<11, 4>(a, f, batch, s));
+            e = mb == 2 ? br_fft_mb_launch<11, 2>(a, f, most, s)
+                        : (mb == 3 ? br_fft_mb_launch<11, 3>(a, f, most, s) : br_fft_mb_launch<11, 4>(a, f, most, s));
             break;
         default: return cudaErrorInvalidValue;
+    }
+    if (e == cudaSuccess && rest) {
+        BlindRotateArgs t = a;
+        t.a += static_cast<size_t>(most) * a.a_stride;
+        t.b += most;
+        t.mv_out += static_cast<size_t>(most) * a.num_lut * 2 * N;
+        e = launch_blind_rotate_fft_solo(t, f, N, rest, s);
     }
     if (e != cudaSuccess || !mv_ntt) return e;
     return ntt_forward(a.mv_out, a.mv_out, a.t.rp, a.t.rps, d_mod, N, static_cast<size_t>(batch) * a.num_lut * 2, s);

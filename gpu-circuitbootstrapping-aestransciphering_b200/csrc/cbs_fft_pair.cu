@@ -1,0 +1,102 @@
+// cbs_fft_pair.cu -- the CBS blind rotation (FP64 FFT, mb = 2, N = 2048, three digits) of two
+// ciphertexts per CTA (br_pair.cuh): k_blind_rotate_fft_mb's arithmetic (offset-form accumulator mod
+// Q), finalize and multi-value split.  2^12 x 3 at 296 ciphertexts: 7.72 -> 4.64 ms against the
+// digit-by-digit kernel (26.1 -> 15.7 us per bootstrap).  Two digits keep k_blind_rotate_fft_mb2_x2
+// (3.43 ms; this form 3.50-3.63).  An odd batch's last CTA runs its second ciphertext as a copy
+// of the first and writes nothing for it.
+#include "common.cuh"
+#include "br_pair.cuh"
+#include "fft_kernels.cuh"
+
+namespace cbs {
+
+struct PairCbsAcc {
+    using Word = int64_t;  // y = centre(x) + round_c in [lo, hi)
+    const FftKeyArgs& f;
+    int ign, gbits;
+    uint32_t fmask;
+    DigitBias bias;
+    int64_t lo, hi, Q;
+    __device__ __forceinline__ double digit(int64_t y, int d) const {
+        return bias(static_cast<uint32_t>(static_cast<uint64_t>(y) >> (ign + gbits * d)) & fmask);
+    }
+    __device__ __forceinline__ int64_t add(int64_t y, double v) const {
+        return offset_add(y, centred_residue(v * f.inv_m, f), lo, hi, Q);
+    }
+};
+
+template <int LOGN, int DIG>
+__global__ void __launch_bounds__(512, 1)
+    k_blind_rotate_fft_pair(const BlindRotateArgs a, const FftKeyArgs f, uint32_t batch) {
+    using Th = PairThread<LOGN, DIG, 2>;
+    using Cfg = typename Th::Cfg;
+    constexpr uint32_t N = Cfg::N, TWO_N = 2 * N;
+    extern __shared__ __align__(16) uint8_t pair_sm[];
+    Th th(pair_sm, a.n);
+    const uint64_t Q = a.t.q, qhalf = Q >> 1;
+    const int gbits = a.g.gbits, ign = a.g.ign;
+    int64_t offset = 0;
+    for (int k = 0; k < DIG; ++k) offset += static_cast<int64_t>(1) << (gbits * k + gbits - 1);
+    const uint64_t round_c = (ign ? (uint64_t(1) << (ign - 1)) : 0) + (static_cast<uint64_t>(offset) << ign);
+    const int64_t hi = static_cast<int64_t>(round_c + qhalf), Qs = static_cast<int64_t>(Q), lo = hi - Qs;
+    const uint32_t ct0 = blockIdx.x * Cfg::CTS + 2 * th.set;
+    auto ct_of = [&](uint32_t c) { return ct0 + c < batch ? ct0 + c : batch - 1; };
+    const uint32_t ct = ct_of(th.c2);
+    const bool live = ct0 + th.c2 < batch;
+    pair_begin(th, pair_sm, f.tab);
+    {
+        // polynomial 0 = 0, polynomial 1 = X^b times the test vector, in offset form
+        const uint32_t bt = special_ms_f(a.b[ct], TWO_N, a.q_lwe, a.bitwidth);
+        auto to_offset = [&](uint64_t x) { return static_cast<int64_t>(x + round_c) - (x >= qhalf ? Qs : 0); };
+        pair_init<int64_t>(th, [&](uint32_t i) -> int64_t {
+            if (th.h == 0) return to_offset(0);
+            const uint32_t s = (i + bt) & (TWO_N - 1);
+            const uint64_t v = (s < N) ? a.tv[s] : a.tv[s - N];
+            return to_offset((s < N) ? v : (v ? Q - v : 0));
+        });
+    }
+    const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
+    pair_rotations(th, a.n, [&](uint32_t i) { return special_ms_f(__ldg(arow + i), TWO_N, a.q_lwe, a.bitwidth); });
+    __syncthreads();
+    const PairCbsAcc acc{f, ign, gbits, (1u << gbits) - 1u, DigitBias(1u << (gbits - 1)), lo, hi, Qs};
+    pair_groups<LOGN, DIG>(th, acc, f.bskf, a.n);
+    // the accumulator to shared memory (natural order, each row in its exchange buffers), finalize,
+    // and the MV split, as in the one-bit form
+    __syncthreads();
+    uint64_t* x = reinterpret_cast<uint64_t*>(th.buf);
+    pair_read<int64_t>(th, [&](uint32_t e, int64_t y) {
+        const int64_t v0 = y - static_cast<int64_t>(round_c);
+        uint64_t v = mul_shoup(static_cast<uint64_t>(v0 < 0 ? v0 + Qs : v0), a.t.n_inv, a.t.n_inv_s, Q);
+        if (th.h == 1 && e < a.num_lut) v = add_mod(v, a.gadd[e], Q);
+        x[e] = v;
+    });
+    pair_end(th);
+    if (!live) return;
+    for (uint32_t j = 0; j < a.num_lut; ++j) {
+        uint64_t* dst = a.mv_out + ((static_cast<size_t>(ct) * a.num_lut + j) * 2 + th.h) * N;
+        for (uint32_t i = th.ht; i < N; i += Cfg::TH) {
+            const uint32_t s = i + j;
+            dst[i] = (s < N) ? x[s] : (x[s - N] ? Q - x[s - N] : 0);
+        }
+    }
+}
+
+cudaError_t launch_blind_rotate_fft_pair3(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch,
+                                          cudaStream_t s) {
+    using Cfg = PairCfg<11, 3, 2>;
+    if (f.tab_len != Cfg::Tb::size()) return cudaErrorInvalidValue;
+    const size_t smem = Cfg::smem(a.n);
+    static size_t configured[64] = {};  // per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (configured[dev] < smem) {
+        cudaError_t e = cudaFuncSetAttribute(k_blind_rotate_fft_pair<11, 3>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        configured[dev] = smem;
+    }
+    k_blind_rotate_fft_pair<11, 3><<<(batch + Cfg::CTS - 1) / Cfg::CTS, Cfg::T, smem, s>>>(a, f, batch);
+    return cudaGetLastError();
+}
+
+}  // namespace cbs

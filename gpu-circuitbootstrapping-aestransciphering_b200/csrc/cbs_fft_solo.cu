@@ -2,9 +2,8 @@
 // CTA or per cluster of two (br_solo.cuh); k_blind_rotate_fft_mb's arithmetic (offset-form
 // accumulator mod Q), finalize and multi-value split.
 //
-// Measured at N = 2048, n = 630, 2^18 x 2: 1-74 ciphertexts 1.98 ms (clusters of two), 75-148
-// 2.49 ms (one CTA each), against 2.90 ms lockstep and 3.40 ms paired; 149 up go to the paired form
-// (3.43 ms for 296, where two waves of this one would take 4.98).
+// Measured at N = 2048, n = 630, 2^18 x 2: 1-74 ciphertexts 1.89 ms (clusters of two), 75-148
+// 2.42 ms (one CTA each), against 2.90 ms lockstep and 3.40 ms paired.
 #include "common.cuh"
 #include "br_solo.cuh"
 #include "fft_kernels.cuh"
@@ -52,10 +51,11 @@ __global__ void __launch_bounds__(512, 1) k_blind_rotate_fft_solo(const BlindRot
     }
     CbsAcc<Cfg::M> acc{y, f, ign, gbits, (1u << gbits) - 1u, DigitBias(1u << (gbits - 1)), lo, hi, Qs};
     const uint64_t* arow = a.a + static_cast<size_t>(ct) * a.a_stride;
+    uint16_t* rot = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(solo_sm) + Cfg::rot_off(8));
+    for (uint32_t i = tid; i < ((a.n + 1) & ~1u); i += Cfg::T)
+        rot[i] = static_cast<uint16_t>(i < a.n ? special_ms_f(__ldg(arow + i), TWO_N, a.q_lwe, a.bitwidth) : 0u);
     solo_sync<CL>();
-    solo_groups<LOGN, DIG, CL>(solo_sm, acc, f.bskf, (a.n + 1) / 2, [&](uint32_t i) {
-        return i < a.n ? special_ms_f(__ldg(arow + i), TWO_N, a.q_lwe, a.bitwidth) : 0u;
-    });
+    solo_groups<LOGN, DIG, CL>(solo_sm, acc, f.bskf, (a.n + 1) / 2, rot);
     // finalize and the MV split, as in the one-bit form
     uint64_t* x = reinterpret_cast<uint64_t*>(y);
     for (uint32_t i = tid; i < Cfg::POLYS * N; i += Cfg::T) {
@@ -79,20 +79,36 @@ template <int LOGN, int DIG>
 static cudaError_t br_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch, uint32_t cl, cudaStream_t s) {
     if (f.tab_len != FftTab<LOGN - 1>::size()) return cudaErrorInvalidValue;
     if (cl == 2)
-        return solo_launch<2>(k_blind_rotate_fft_solo<LOGN, DIG, 2>, 2 * batch, SoloCfg<LOGN, DIG, 2>::smem(8), s, a, f);
-    return solo_launch<1>(k_blind_rotate_fft_solo<LOGN, DIG, 1>, batch, SoloCfg<LOGN, DIG, 1>::smem(8), s, a, f);
+        return solo_launch<2>(k_blind_rotate_fft_solo<LOGN, DIG, 2>, 2 * batch, SoloCfg<LOGN, DIG, 2>::smem(8, a.n), s, a, f);
+    return solo_launch<1>(k_blind_rotate_fft_solo<LOGN, DIG, 1>, batch, SoloCfg<LOGN, DIG, 1>::smem(8, a.n), s, a, f);
 }
 
 cudaError_t launch_blind_rotate_fft_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t batch,
-                                         cudaStream_t s, bool* taken) {
-    *taken = false;
-    if ((a.digits != 2 && a.digits != 3) || (N != 1024 && N != 2048)) return cudaSuccess;
+                                         cudaStream_t s) {
     uint32_t cl = 0;
     cudaError_t e = solo_ctas(batch, &cl);
-    if (e != cudaSuccess || cl == 0) return e;
-    *taken = true;
+    if (e != cudaSuccess) return e;
     if (N == 1024) return a.digits == 2 ? br_solo<10, 2>(a, f, batch, cl, s) : br_solo<10, 3>(a, f, batch, cl, s);
     return a.digits == 2 ? br_solo<11, 2>(a, f, batch, cl, s) : br_solo<11, 3>(a, f, batch, cl, s);
+}
+
+// A wave of the throughput form takes as long for one ciphertext as for per_sm of them on every SM; a
+// wave of the small-batch form (one per SM) takes 0.37 (N = 1024 gates: 1.67 of 4.48 ms, four per SM)
+// to 0.71 (CBS 2 x 18 bits: 2.42 of 3.43 ms, two per SM) of that.  So what the last wave would leave
+// goes to the small-batch form while it fills no more than half of a wave.
+cudaError_t solo_rest(uint32_t batch, uint32_t per_sm, uint32_t* rest) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const uint32_t n = static_cast<uint32_t>(sms);
+    if (per_sm == 0) {
+        *rest = batch <= n ? batch : 0;
+    } else {
+        const uint32_t r = batch % (per_sm * n);
+        *rest = r <= per_sm * n / 2 ? r : 0;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace cbs

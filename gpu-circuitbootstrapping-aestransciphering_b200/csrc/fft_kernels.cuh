@@ -100,10 +100,15 @@ cudaError_t launch_blind_rotate_fft(const BlindRotateArgs& a, const FftKeyArgs& 
 // [ceil(n/mb)][2^mb - 1][2*digits][2][N/2]
 cudaError_t launch_blind_rotate_fft_mb(const BlindRotateArgs& a, const FftKeyArgs& f, const cbs_dmodulus* d_mod,
                                        uint32_t N, uint32_t batch, uint32_t mb, cudaStream_t s, bool mv_ntt = true);
-// the small-batch form of mb = 2 (cbs_fft_solo.cu); *taken = false, nothing launched, where it does
-// not apply
+// two ciphertexts per CTA: mb = 2, N = 2048, three digits (cbs_fft_pair.cu)
+cudaError_t launch_blind_rotate_fft_pair3(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t batch,
+                                          cudaStream_t s);
+// the small-batch form of mb = 2, two or three digits, N = 1024 or 2048 (cbs_fft_solo.cu)
 cudaError_t launch_blind_rotate_fft_solo(const BlindRotateArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t batch,
-                                         cudaStream_t s, bool* taken);
+                                         cudaStream_t s);
+// ciphertexts at the end of a batch that take the small-batch form, beside a throughput form of
+// `per_sm` ciphertexts per SM (0: only whole batches up to the SM count)
+cudaError_t solo_rest(uint32_t batch, uint32_t per_sm, uint32_t* rest);
 cudaError_t launch_trace_ss_fft(const TraceFftArgs& a, const FftKeyArgs& f, uint32_t N, uint32_t count, cudaStream_t s);
 // digit spectra of the pair differences of `sets` fixed level-0 input sets (a.in, a.in_lut_stride,
 // a.in_count, a.g, a.digits) into out [sets][in_count/2][2*digits][N/2]

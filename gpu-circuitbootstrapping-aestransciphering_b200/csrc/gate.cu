@@ -635,9 +635,19 @@ static cudaError_t gate_br_dispatch(const GateArgs& a, uint32_t N, uint32_t grid
         if (N == 2048) return gate_br_launch<11, TT>(a, grid, s);
         return cudaErrorInvalidValue;
     }
-    bool solo = false;
-    const cudaError_t se = gate_blind_rotate_solo<TT>(a, N, s, &solo);
-    if (solo || se != cudaSuccess) return se;
+    if (a.mb == 2 && (a.levels == 2 || a.levels == 3) && (N == 1024 || N == 2048)) {
+        // two ciphertexts per lane set, what a wave leaves over one per CTA; a persistent grid the
+        // caller asked for is kept for the whole batch
+        uint32_t rest = 0;
+        cudaError_t e = grid < a.items ? cudaSuccess : solo_rest(a.items, N == 1024 ? 4 : 2, &rest);
+        GateArgs t = a;
+        t.items = a.items - rest;
+        if (e == cudaSuccess && t.items) e = gate_blind_rotate_pair<TT>(t, N, grid, s);
+        t.item0 = t.items;
+        t.items = a.items;
+        if (e == cudaSuccess && rest) e = gate_blind_rotate_solo<TT>(t, N, s);
+        return e;
+    }
     if (a.mb == 2) {
         if (N == 1024) return gate_br_mb_launch<10, TT, 2>(a, grid, s);
         if (N == 2048) return gate_br_mb_launch<11, TT, 2>(a, grid, s);

@@ -1,0 +1,102 @@
+// gate_pair.cu -- the torus blind rotation (gates, torus circuit bootstrap; mb = 2, two or three
+// levels) of two ciphertexts per lane set (br_pair.cuh): two per CTA at N = 2048, four at N = 1024.
+// The products round to the same integers as k_gate_blind_rotate_mb's, so the 32-bit results are the
+// same words.  Rows past the last item run a copy of it and write nothing.
+#include "common.cuh"
+#include "br_pair.cuh"
+#include "gate_ops.cuh"
+
+namespace cbs {
+
+template <typename TT, uint32_t M>
+struct PairTorusAcc {
+    using Word = TT;
+    TT off;
+    uint32_t bg, fmask;
+    DigitBias bias;
+    __device__ __forceinline__ double digit(TT y, int d) const {
+        const uint32_t sft = 8 * sizeof(TT) - (static_cast<uint32_t>(d) + 1) * bg;
+        return bias(static_cast<uint32_t>((y + off) >> sft) & fmask);
+    }
+    __device__ __forceinline__ TT add(TT y, double v) const {
+        constexpr double inv_m = 1.0 / M;
+        return y + to_torus<TT>(v * inv_m);
+    }
+};
+
+template <int LOGN, int DIG, typename TT>
+__global__ void __launch_bounds__(512, 1) k_gate_pair(const GateArgs a) {
+    using Th = PairThread<LOGN, DIG, sizeof(TT) / 4>;
+    using Cfg = typename Th::Cfg;
+    constexpr uint32_t N = Cfg::N, TWO_N = 2 * N, SH = 32 - (LOGN + 1), W = 8 * sizeof(TT);
+    extern __shared__ __align__(16) uint8_t pair_sm[];
+    Th th(pair_sm, a.n);
+    pair_begin(th, pair_sm, a.tab);
+    auto ms = [](uint32_t x) { return ((x + (1u << (SH - 1))) >> SH) & (TWO_N - 1); };
+    TT off = TT(1) << (W - DIG * a.bg_bits - 1);
+    for (uint32_t k = 0; k < DIG; ++k) off += (TT(1) << (a.bg_bits - 1)) << (W - (k + 1) * a.bg_bits);
+    const PairTorusAcc<TT, Cfg::M> acc{off, a.bg_bits, (1u << a.bg_bits) - 1u, DigitBias(1u << (a.bg_bits - 1))};
+    for (uint32_t base = blockIdx.x * Cfg::CTS; base < a.items; base += gridDim.x * Cfg::CTS) {
+        const uint32_t it = base + 2 * th.set + th.c2, mine = it < a.items ? it : a.items - 1;
+        const uint32_t *a1, *a2;
+        uint32_t b;
+        gate_item_inputs(a, mine, a1, a2, b);
+        pair_rotations(th, a.n, [&](uint32_t i) {
+            return ms(a.reqs ? __ldg(a1 + i) : gate_a(a.gate, __ldg(a1 + i), __ldg(a2 + i)));
+        });
+        {
+            const uint32_t bt = ms(b);
+            const TT mu = static_cast<TT>(a.mu[mine % a.levels_tv]);
+            pair_init<TT>(th, [&](uint32_t i) -> TT {
+                if (th.h == 0) return 0;
+                const uint32_t sp = (i + bt) & (TWO_N - 1);
+                const TT tv = a.tv ? static_cast<TT>(__ldg(a.tv + (sp & (N - 1)))) : mu;
+                return sp < N ? tv : TT(0) - tv;
+            });
+        }
+        __syncthreads();
+        pair_groups<LOGN, DIG>(th, acc, a.bskf, a.n);
+        // sample extract of coefficient 0: a'_0 = a_0, a'_i = -a_(N-i), b' = b_0
+        __syncthreads();
+        TT* x = reinterpret_cast<TT*>(th.buf);
+        pair_read<TT>(th, [&](uint32_t e, TT v) { x[e] = v; });
+        __syncthreads();
+        if (it < a.items) {
+            TT* out = reinterpret_cast<TT*>(a.ext) + static_cast<size_t>(mine) * (N + 1);
+            if (th.h == 0)
+                for (uint32_t i = th.ht; i < N; i += Cfg::TH) out[i] = i == 0 ? x[0] : TT(0) - x[N - i];
+            else if (th.ht == 0) out[N] = x[0] + static_cast<TT>(a.b_add[mine % a.levels_tv]);
+        }
+        __syncthreads();
+    }
+    pair_end(th);
+}
+
+template <int LOGN, int DIG, typename TT>
+static cudaError_t gate_pair(const GateArgs& a, uint32_t grid, cudaStream_t s) {
+    using Cfg = PairCfg<LOGN, DIG, sizeof(TT) / 4>;
+    const size_t smem = Cfg::smem(a.n);
+    static size_t configured[64] = {};  // per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (configured[dev] < smem) {
+        cudaError_t e = cudaFuncSetAttribute(k_gate_pair<LOGN, DIG, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        configured[dev] = smem;
+    }
+    // a persistent grid of `grid` single-ciphertext CTAs becomes one of grid / CTS
+    const uint32_t items = grid < a.items ? grid : a.items;
+    k_gate_pair<LOGN, DIG, TT><<<(items + Cfg::CTS - 1) / Cfg::CTS, Cfg::T, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+template <typename TT>
+cudaError_t gate_blind_rotate_pair(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s) {
+    if (N == 1024) return a.levels == 2 ? gate_pair<10, 2, TT>(a, grid, s) : gate_pair<10, 3, TT>(a, grid, s);
+    return a.levels == 2 ? gate_pair<11, 2, TT>(a, grid, s) : gate_pair<11, 3, TT>(a, grid, s);
+}
+template cudaError_t gate_blind_rotate_pair<uint32_t>(const GateArgs&, uint32_t, uint32_t, cudaStream_t);
+template cudaError_t gate_blind_rotate_pair<uint64_t>(const GateArgs&, uint32_t, uint32_t, cudaStream_t);
+
+}  // namespace cbs

@@ -2,8 +2,8 @@
 // ciphertext per CTA or per cluster of two (br_solo.cuh); the products round to the same integers as
 // k_gate_blind_rotate_mb's, so the 32-bit results are the same words.
 //
-// Measured, grouped mb = 2: 64 gates (n = 636, N = 1024; clusters of two) 2.88 -> 1.51 ms, 144
-// level-2 rotations (n = 630, N = 2048, 64-bit torus; one CTA each) 3.85 -> 3.3 ms.
+// Measured, grouped mb = 2: 64 gates (n = 636, N = 1024; clusters of two) 2.88 -> 1.41 ms, 148
+// bootstraps at N = 2048 (n = 630; one CTA each) 3.8 -> 2.97 ms.
 #include "common.cuh"
 #include "br_solo.cuh"
 #include "gate_ops.cuh"
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(512, 1) k_gate_solo(const GateArgs a) {
     using Cfg = SoloCfg<LOGN, DIG, CL>;
     constexpr uint32_t N = Cfg::N, TWO_N = 2 * N, SH = 32 - (LOGN + 1), W = 8 * sizeof(TT);
     extern __shared__ __align__(16) double2 solo_sm[];
-    const uint32_t tid = threadIdx.x, rank = solo_rank<CL>(), item = blockIdx.x / CL;
+    const uint32_t tid = threadIdx.x, rank = solo_rank<CL>(), item = a.item0 + blockIdx.x / CL;
     for (uint32_t i = tid; i < Cfg::Tb::size(); i += Cfg::T) solo_sm[i] = a.tab[i];
     auto ms = [](uint32_t x) { return ((x + (1u << (SH - 1))) >> SH) & (TWO_N - 1); };
     const uint32_t *a1, *a2;
@@ -53,10 +53,12 @@ __global__ void __launch_bounds__(512, 1) k_gate_solo(const GateArgs a) {
         accp[i] = poly == 0 ? TT(0) : (sp < N ? tv : TT(0) - tv);
     }
     TorusAcc<TT, Cfg::M> acc{accp, off, a.bg_bits, (1u << a.bg_bits) - 1u, DigitBias(1u << (a.bg_bits - 1))};
+    uint16_t* rot = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(solo_sm) + Cfg::rot_off(sizeof(TT)));
+    for (uint32_t i = tid; i < ((a.n + 1) & ~1u); i += Cfg::T)
+        rot[i] = static_cast<uint16_t>(
+            i < a.n ? ms(a.reqs ? __ldg(a1 + i) : gate_a(a.gate, __ldg(a1 + i), __ldg(a2 + i))) : 0u);
     solo_sync<CL>();
-    solo_groups<LOGN, DIG, CL>(solo_sm, acc, a.bskf, (a.n + 1) / 2, [&](uint32_t i) {
-        return i < a.n ? ms(a.reqs ? __ldg(a1 + i) : gate_a(a.gate, __ldg(a1 + i), __ldg(a2 + i))) : 0u;
-    });
+    solo_groups<LOGN, DIG, CL>(solo_sm, acc, a.bskf, (a.n + 1) / 2, rot);
     // sample extract of coefficient 0: a'_0 = a_0, a'_i = -a_(N-i), b' = b_0
     TT* out = reinterpret_cast<TT*>(a.ext) + static_cast<size_t>(item) * (N + 1);
     if (rank == 0)
@@ -66,23 +68,21 @@ __global__ void __launch_bounds__(512, 1) k_gate_solo(const GateArgs a) {
 
 template <int LOGN, int DIG, typename TT>
 static cudaError_t gate_solo(const GateArgs& a, uint32_t cl, cudaStream_t s) {
+    const uint32_t count = a.items - a.item0;
     if (cl == 2)
-        return solo_launch<2>(k_gate_solo<LOGN, DIG, 2, TT>, 2 * a.items, SoloCfg<LOGN, DIG, 2>::smem(sizeof(TT)), s, a);
-    return solo_launch<1>(k_gate_solo<LOGN, DIG, 1, TT>, a.items, SoloCfg<LOGN, DIG, 1>::smem(sizeof(TT)), s, a);
+        return solo_launch<2>(k_gate_solo<LOGN, DIG, 2, TT>, 2 * count, SoloCfg<LOGN, DIG, 2>::smem(sizeof(TT), a.n), s, a);
+    return solo_launch<1>(k_gate_solo<LOGN, DIG, 1, TT>, count, SoloCfg<LOGN, DIG, 1>::smem(sizeof(TT), a.n), s, a);
 }
 
 template <typename TT>
-cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s, bool* taken) {
-    *taken = false;
-    if (a.mb != 2 || a.fft_mode != 0 || (a.levels != 2 && a.levels != 3) || (N != 1024 && N != 2048)) return cudaSuccess;
+cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s) {
     uint32_t cl = 0;
-    cudaError_t e = solo_ctas(a.items, &cl);
-    if (e != cudaSuccess || cl == 0) return e;
-    *taken = true;
+    cudaError_t e = solo_ctas(a.items - a.item0, &cl);
+    if (e != cudaSuccess) return e;
     if (N == 1024) return a.levels == 2 ? gate_solo<10, 2, TT>(a, cl, s) : gate_solo<10, 3, TT>(a, cl, s);
     return a.levels == 2 ? gate_solo<11, 2, TT>(a, cl, s) : gate_solo<11, 3, TT>(a, cl, s);
 }
-template cudaError_t gate_blind_rotate_solo<uint32_t>(const GateArgs&, uint32_t, cudaStream_t, bool*);
-template cudaError_t gate_blind_rotate_solo<uint64_t>(const GateArgs&, uint32_t, cudaStream_t, bool*);
+template cudaError_t gate_blind_rotate_solo<uint32_t>(const GateArgs&, uint32_t, cudaStream_t);
+template cudaError_t gate_blind_rotate_solo<uint64_t>(const GateArgs&, uint32_t, cudaStream_t);
 
 }  // namespace cbs

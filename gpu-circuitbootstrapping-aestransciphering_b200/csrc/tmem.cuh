@@ -69,6 +69,21 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
         : "memory");
 }
 
+// four columns into r[0..3], without the wait (tmem_wait_load before r is used)
+__device__ __forceinline__ void tmem_load4_nowait(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+template <int COUNT>
+__device__ __forceinline__ void tmem_wait_load(uint32_t (&r)[COUNT][4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < COUNT; ++k)  // later uses of r stay behind the wait
+        asm volatile("" : "+r"(r[k][0]), "+r"(r[k][1]), "+r"(r[k][2]), "+r"(r[k][3]));
+}
+
 // one complex value in four columns
 __device__ __forceinline__ void tmem_store_complex(uint32_t taddr, double2 a) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr),

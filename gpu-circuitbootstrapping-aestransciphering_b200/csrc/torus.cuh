@@ -36,6 +36,7 @@ struct GateArgs {
     const GateReq* reqs;   // ragged mode when non-null: items are the concatenated requests
     uint32_t num_reqs;
     uint32_t items;        // ciphertexts in total; CTAs loop over them with stride gridDim.x
+    uint32_t item0;        // first ciphertext of the launch (the small-batch kernel only; else 0)
     // test vectors: item i rotates the constant test vector mu[i % levels_tv] of input
     // i / levels_tv and adds b_add[i % levels_tv] to the extracted b (gates: one level, 1/8, 0)
     uint32_t levels_tv;
@@ -56,9 +57,12 @@ struct GateArgs {
 
 cudaError_t gate_blind_rotate(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);    // 32-bit torus
 cudaError_t gate_blind_rotate64(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);  // 64-bit torus
-// the small-batch form (gate_solo.cu); *taken = false, nothing launched, where it does not apply
+// mb = 2 with two or three levels, FP64: the small-batch form for items [a.item0, a.items)
+// (gate_solo.cu) and the throughput form (gate_pair.cu)
 template <typename TT>
-cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s, bool* taken);
+cudaError_t gate_blind_rotate_solo(const GateArgs& a, uint32_t N, cudaStream_t s);
+template <typename TT>
+cudaError_t gate_blind_rotate_pair(const GateArgs& a, uint32_t N, uint32_t grid, cudaStream_t s);
 
 uint32_t torus_from_double(double x);
 uint32_t torus_noise(Rng& rng, double sigma);

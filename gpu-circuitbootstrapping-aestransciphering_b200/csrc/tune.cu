@@ -216,7 +216,8 @@ cbs_status cbs_autotune_blind_rotation(cbs_context* ctx, uint32_t batch, const c
         if (cbs_status st = cbs_context_set_br_multibit(c, mb)) return st;
         std::vector<uint32_t> schedules = {CBS_BR_SCHEDULE_DIGITWISE};
         if (mb == 2 && c->p.digits_g == 2) schedules.push_back(CBS_BR_SCHEDULE_LOCKSTEP);
-        if (mb == 2 && c->p.digits_g == 2 && c->p.N == 2048 && batch >= 2) schedules.push_back(CBS_BR_SCHEDULE_PAIRED);
+        if (mb == 2 && (c->p.digits_g == 2 || c->p.digits_g == 3) && c->p.N == 2048 && batch >= 2)
+            schedules.push_back(CBS_BR_SCHEDULE_PAIRED);
         for (uint32_t sch : schedules) {
             c->br_schedule = sch;
             if (cbs_status st = run_blind_rotate(c, d_a.p, d_b.p, batch, c->p.n, c->d_mv.p, s, false)) return st;
