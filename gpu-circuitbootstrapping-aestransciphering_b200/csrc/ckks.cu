@@ -47,7 +47,7 @@ __device__ __forceinline__ uint64_t mod_product(uint64_t a, uint64_t b, const El
     const uint64_t q = __ldg(e.q + l);
     if (e.qinv) {
         const DMod md{static_cast<double>(q), __ldg(e.qinv + l)};
-        return dto_residue(dmulmod(__ull2double_rn(a), __ull2double_rn(b), md), md);
+        return dto_residue(dmulmod(dfrom_u52(a), dfrom_u52(b), md), md);
     }
     return barrett_reduce_128(mul_wide(a, b), q, __ldg(e.r0 + l), __ldg(e.r1 + l));
 }

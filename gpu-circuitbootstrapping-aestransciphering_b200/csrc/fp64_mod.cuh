@@ -6,7 +6,9 @@
 // computed exactly in doubles:
 //   h = fl(v w), l = fma(v, w, -h)          (error-free product, Ogita-Rump-Oishi TwoProduct:
 //                                            v w = h + l exactly)
-//   k = rint(h * fl(1/q))                   (quotient estimate: |v w / q - k| <= 1/2 + 3 |v| 2^-53)
+//   k = rint(h * fl(1/q))                   (quotient estimate: |v w / q - k| <= 1/2 + 3 |v| 2^-53;
+//                                            rounded by adding and subtracting 1.5 2^52, which
+//                                            runs at the full FP64 rate, and rint does not)
 //   r = fma(-k, q, h) + l                    (= v w - k q exactly)
 // fma(-k, q, h) is exact because its true value h - k q = r - l is an integer below 2^53 in
 // magnitude; r is congruent to v w and |r| <= q (1/2 + 3 |v| 2^-53), i.e. below 0.875 q for
@@ -24,24 +26,40 @@ struct DMod {
 
 __device__ __forceinline__ DMod dmod_of(uint64_t q) { return {static_cast<double>(q), 1.0 / static_cast<double>(q)}; }
 
-// v w mod q, signed (see above), exact for |v| < 2^52 and 0 <= w < q < 2^50
+// the nearest integer to a b, |a b| < 2^51
+__device__ __forceinline__ double dround_product(double a, double b) {
+    constexpr double c = 0x1.8p52;
+    return __dadd_rn(__fma_rn(a, b, c), -c);
+}
+
+// v w mod q, signed (see above), exact for |v| < 2^52 and |w| < q < 2^50 with |v w| / q < 2^51: any
+// |v| <= 2q + 4, or |v| <= 4q + 8 with w centred (|w| <= q / 2)
 __device__ __forceinline__ double dmulmod(double v, double w, const DMod& m) {
     const double h = __dmul_rn(v, w);
     const double l = __fma_rn(v, w, -h);
-    const double k = rint(__dmul_rn(h, m.qinv));
+    const double k = dround_product(h, m.qinv);
     return __dadd_rn(__fma_rn(-k, m.q, h), l);
 }
 
-// x mod q in [-q/2 - 1, q/2 + 1] for |x| < 2^53
+// x mod q in [-q/2 - 1, q/2 + 1] for |x| < 2^53, |x| / q < 2^51
 __device__ __forceinline__ double dreduce(double x, const DMod& m) {
-    return __fma_rn(-rint(__dmul_rn(x, m.qinv)), m.q, x);
+    return __fma_rn(-dround_product(x, m.qinv), m.q, x);
+}
+
+// integers below 2^52 to and from FP64 through the mantissa of 2^52 + v (one addition, where the
+// conversion instructions run at a quarter of the FP64 rate)
+__device__ __forceinline__ double dfrom_u52(uint64_t v) {
+    return __dadd_rn(__longlong_as_double(static_cast<long long>(v | 0x4330000000000000ull)), -0x1p52);
+}
+__device__ __forceinline__ uint64_t dto_u52(double r) {
+    return static_cast<uint64_t>(__double_as_longlong(__dadd_rn(r, 0x1p52))) & 0xfffffffffffffull;
 }
 
 // the residue in [0, q) of an integer |x| < 2^53
 __device__ __forceinline__ uint64_t dto_residue(double x, const DMod& m) {
     double r = dreduce(x, m);
     if (r < 0.0) r = __dadd_rn(r, m.q);
-    return __double2ull_rn(r);
+    return dto_u52(r);
 }
 
 }  // namespace cbs

@@ -75,105 +75,106 @@ __device__ __forceinline__ uint32_t pass_group(uint32_t m, uint32_t tid, int set
     return (4 * tid + set) / (N / (2 * m));
 }
 
+// A thread's twiddles (and Shoup quotients) of one pass, group index base + k (base = m for a whole
+// transform):
+//   three stages: [i1] [2 i1, 2 i1 + 1] [4 i1 .. 4 i1 + 3]; two: per set [i1] [2 i1, 2 i1 + 1]; one: [i1] per set
+struct TwU {
+    uint64_t w[7], s[7];
+};
 template <int LOGN, int R>
-__device__ __forceinline__ void fwd_pass(uint64_t (&x)[8], uint32_t m, uint32_t tid, const uint64_t* __restrict__ tw,
-                                         const uint64_t* __restrict__ tws, uint64_t q) {
-    const uint64_t q2 = q << 1;
+__device__ __forceinline__ TwU load_tw(uint32_t m, uint32_t base, uint32_t tid, const uint64_t* __restrict__ tw,
+                                       const uint64_t* __restrict__ tws) {
+    TwU t;
+    auto get = [&](int at, uint32_t i) {
+        t.w[at] = __ldg(tw + i);
+        t.s[at] = __ldg(tws + i);
+    };
     if (R == 3) {
-        const uint32_t k = pass_group<LOGN, 3>(m, tid, 0);
-        const uint32_t i1 = m + k;
-        {
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
+        const uint32_t i1 = base + pass_group<LOGN, 3>(m, tid, 0);
+        get(0, i1);
+        get(1, 2 * i1);
+        get(2, 2 * i1 + 1);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) ct_bf(x[j], x[j + 4], w, ws, q2, q);
-        }
-        {
-            const uint64_t w0 = __ldg(tw + 2 * i1), w0s = __ldg(tws + 2 * i1);
-            const uint64_t w1 = __ldg(tw + 2 * i1 + 1), w1s = __ldg(tws + 2 * i1 + 1);
-            ct_bf(x[0], x[2], w0, w0s, q2, q);
-            ct_bf(x[1], x[3], w0, w0s, q2, q);
-            ct_bf(x[4], x[6], w1, w1s, q2, q);
-            ct_bf(x[5], x[7], w1, w1s, q2, q);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t ti = 4 * i1 + j;
-            ct_bf(x[2 * j], x[2 * j + 1], __ldg(tw + ti), __ldg(tws + ti), q2, q);
-        }
+        for (int j = 0; j < 4; ++j) get(3 + j, 4 * i1 + j);
     } else if (R == 2) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint32_t k = pass_group<LOGN, 2>(m, tid, h);
-            const uint32_t i1 = m + k;
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-            uint64_t* v = x + 4 * h;
-            ct_bf(v[0], v[2], w, ws, q2, q);
-            ct_bf(v[1], v[3], w, ws, q2, q);
-            ct_bf(v[0], v[1], __ldg(tw + 2 * i1), __ldg(tws + 2 * i1), q2, q);
-            ct_bf(v[2], v[3], __ldg(tw + 2 * i1 + 1), __ldg(tws + 2 * i1 + 1), q2, q);
+            const uint32_t i1 = base + pass_group<LOGN, 2>(m, tid, h);
+            get(3 * h, i1);
+            get(3 * h + 1, 2 * i1);
+            get(3 * h + 2, 2 * i1 + 1);
         }
     } else {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t k = pass_group<LOGN, 1>(m, tid, h);
-            const uint32_t i1 = m + k;
-            ct_bf(x[2 * h], x[2 * h + 1], __ldg(tw + i1), __ldg(tws + i1), q2, q);
+        for (int h = 0; h < 4; ++h) get(h, base + pass_group<LOGN, 1>(m, tid, h));
+    }
+    return t;
+}
+
+template <int R>
+__device__ __forceinline__ void fwd_pass_t(uint64_t (&x)[8], const TwU& t, uint64_t q) {
+    const uint64_t q2 = q << 1;
+    auto bf = [&](uint64_t& u, uint64_t& v, int k) { ct_bf(u, v, t.w[k], t.s[k], q2, q); };
+    if (R == 3) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bf(x[j], x[j + 4], 0);
+        bf(x[0], x[2], 1);
+        bf(x[1], x[3], 1);
+        bf(x[4], x[6], 2);
+        bf(x[5], x[7], 2);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bf(x[2 * j], x[2 * j + 1], 3 + j);
+    } else if (R == 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint64_t* v = x + 4 * h;
+            bf(v[0], v[2], 3 * h);
+            bf(v[1], v[3], 3 * h);
+            bf(v[0], v[1], 3 * h + 1);
+            bf(v[2], v[3], 3 * h + 2);
         }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) bf(x[2 * h], x[2 * h + 1], h);
     }
 }
 
-template <int LOGN, int R>
-__device__ __forceinline__ void inv_pass(uint64_t (&x)[8], uint32_t m, uint32_t tid, const uint64_t* __restrict__ tw,
-                                         const uint64_t* __restrict__ tws, uint64_t q) {
+template <int R>
+__device__ __forceinline__ void inv_pass_t(uint64_t (&x)[8], const TwU& t, uint64_t q) {
     const uint64_t q2 = q << 1;
+    auto bf = [&](uint64_t& u, uint64_t& v, int k) { gs_bf(u, v, t.w[k], t.s[k], q2, q); };
     if (R == 3) {
-        const uint32_t k = pass_group<LOGN, 3>(m, tid, 0);
-        const uint32_t i1 = m + k;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t ti = 4 * i1 + j;
-            gs_bf(x[2 * j], x[2 * j + 1], __ldg(tw + ti), __ldg(tws + ti), q2, q);
-        }
-        {
-            const uint64_t w0 = __ldg(tw + 2 * i1), w0s = __ldg(tws + 2 * i1);
-            const uint64_t w1 = __ldg(tw + 2 * i1 + 1), w1s = __ldg(tws + 2 * i1 + 1);
-            gs_bf(x[0], x[2], w0, w0s, q2, q);
-            gs_bf(x[1], x[3], w0, w0s, q2, q);
-            gs_bf(x[4], x[6], w1, w1s, q2, q);
-            gs_bf(x[5], x[7], w1, w1s, q2, q);
-        }
-        {
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
+        for (int j = 0; j < 4; ++j) bf(x[2 * j], x[2 * j + 1], 3 + j);
+        bf(x[0], x[2], 1);
+        bf(x[1], x[3], 1);
+        bf(x[4], x[6], 2);
+        bf(x[5], x[7], 2);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) gs_bf(x[j], x[j + 4], w, ws, q2, q);
-        }
+        for (int j = 0; j < 4; ++j) bf(x[j], x[j + 4], 0);
     } else if (R == 2) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint32_t k = pass_group<LOGN, 2>(m, tid, h);
-            const uint32_t i1 = m + k;
             uint64_t* v = x + 4 * h;
-            gs_bf(v[0], v[1], __ldg(tw + 2 * i1), __ldg(tws + 2 * i1), q2, q);
-            gs_bf(v[2], v[3], __ldg(tw + 2 * i1 + 1), __ldg(tws + 2 * i1 + 1), q2, q);
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-            gs_bf(v[0], v[2], w, ws, q2, q);
-            gs_bf(v[1], v[3], w, ws, q2, q);
+            bf(v[0], v[1], 3 * h + 1);
+            bf(v[2], v[3], 3 * h + 2);
+            bf(v[0], v[2], 3 * h);
+            bf(v[1], v[3], 3 * h);
         }
     } else {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t k = pass_group<LOGN, 1>(m, tid, h);
-            const uint32_t i1 = m + k;
-            gs_bf(x[2 * h], x[2 * h + 1], __ldg(tw + i1), __ldg(tws + i1), q2, q);
-        }
+        for (int h = 0; h < 4; ++h) bf(x[2 * h], x[2 * h + 1], h);
     }
 }
 
 // Forward NTT of one polynomial held by the CTA's first NttPlan::T threads.
 // load(i) supplies input coefficient i (< 4q); store(j, i, v) receives the fully reduced
 // output at bit-reversed slot i (register slot j of this thread).  sm: N words of shared memory.  The caller must
-// __syncthreads() before reusing sm.
-template <int LOGN, class Load, class Store>
+// __syncthreads() before reusing sm.  AHEAD: the next pass's twiddles are loaded before the barrier
+// it waits at and the passes are unrolled (a transform alone in its kernel, whose time is the
+// latency of these loads: one transform of 2^16 points 16.4 -> 15.5 us; the fused kernels keep the
+// registers).
+template <int LOGN, bool AHEAD = false, class Load, class Store>
 __device__ __forceinline__ void ntt_forward_cta(uint64_t* sm, uint32_t tid, const uint64_t* __restrict__ tw,
                                                 const uint64_t* __restrict__ tws, uint64_t q, Load load, Store store) {
     using Pl = NttPlan<LOGN>;
@@ -182,7 +183,31 @@ __device__ __forceinline__ void ntt_forward_cta(uint64_t* sm, uint32_t tid, cons
     // first radix-8 pass straight from the loader
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(pass_index<LOGN, 3>(1u, tid, j));
-    fwd_pass<LOGN, 3>(x, 1u, tid, tw, tws, q);
+    fwd_pass_t<3>(x, load_tw<LOGN, 3>(1u, 1u, tid, tw, tws), q);
+    if constexpr (AHEAD) {
+#pragma unroll
+        for (int p = 1; p < Pl::P; ++p) {
+            const uint32_t m = 1u << (3 * p);
+            const TwU t = p < Pl::P - 1 ? load_tw<LOGN, 3>(m, m, tid, tw, tws)
+                                        : load_tw<LOGN, Pl::tail_r>(m, m, tid, tw, tws);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, 3>(m / 8, tid, j))] = x[j];
+            __syncthreads();
+            if (p < Pl::P - 1) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, 3>(m, tid, j))];
+                fwd_pass_t<3>(x, t, q);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, Pl::tail_r>(m, tid, j))];
+                fwd_pass_t<Pl::tail_r>(x, t, q);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    store(j, pass_index<LOGN, Pl::tail_r>(m, tid, j), csub(csub(x[j], q << 1), q));
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, 3>(1u, tid, j))] = x[j];
     __syncthreads();
@@ -192,7 +217,7 @@ __device__ __forceinline__ void ntt_forward_cta(uint64_t* sm, uint32_t tid, cons
         const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, 3>(m, tid, j))];
-        fwd_pass<LOGN, 3>(x, m, tid, tw, tws, q);
+        fwd_pass_t<3>(x, load_tw<LOGN, 3>(m, m, tid, tw, tws), q);
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, 3>(m, tid, j))] = x[j];
         __syncthreads();
@@ -202,7 +227,7 @@ __device__ __forceinline__ void ntt_forward_cta(uint64_t* sm, uint32_t tid, cons
         constexpr uint32_t m = 1u << (3 * (Pl::P - 1));
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, Pl::tail_r>(m, tid, j))];
-        fwd_pass<LOGN, Pl::tail_r>(x, m, tid, tw, tws, q);
+        fwd_pass_t<Pl::tail_r>(x, load_tw<LOGN, Pl::tail_r>(m, m, tid, tw, tws), q);
         const uint64_t q2 = q << 1;
 #pragma unroll
         for (int j = 0; j < 8; ++j) store(j, pass_index<LOGN, Pl::tail_r>(m, tid, j), csub(csub(x[j], q2), q));
@@ -210,8 +235,8 @@ __device__ __forceinline__ void ntt_forward_cta(uint64_t* sm, uint32_t tid, cons
 }
 
 // Inverse NTT (n^-1 included) of one polynomial; load(j, i) supplies bit-reversed slot i
-// (< 2q) for register slot j; store(i, v) receives coefficient i fully reduced.
-template <int LOGN, class Load, class Store>
+// (< 2q) for register slot j; store(i, v) receives coefficient i fully reduced.  AHEAD: as above.
+template <int LOGN, bool AHEAD = false, class Load, class Store>
 __device__ __forceinline__ void ntt_inverse_cta(uint64_t* sm, uint32_t tid, const uint64_t* __restrict__ itw,
                                                 const uint64_t* __restrict__ itws, uint64_t n_inv, uint64_t n_inv_s,
                                                 uint64_t q, Load load, Store store) {
@@ -222,7 +247,33 @@ __device__ __forceinline__ void ntt_inverse_cta(uint64_t* sm, uint32_t tid, cons
         constexpr uint32_t m = 1u << (3 * (Pl::P - 1));
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = load(j, pass_index<LOGN, Pl::tail_r>(m, tid, j));
-        inv_pass<LOGN, Pl::tail_r>(x, m, tid, itw, itws, q);
+        inv_pass_t<Pl::tail_r>(x, load_tw<LOGN, Pl::tail_r>(m, m, tid, itw, itws), q);
+        if constexpr (AHEAD) {
+            TwU t = load_tw<LOGN, 3>(m / 8, m / 8, tid, itw, itws);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, Pl::tail_r>(m, tid, j))] = x[j];
+            __syncthreads();
+#pragma unroll
+            for (int p = Pl::P - 2; p >= 0; --p) {
+                const uint32_t mp = 1u << (3 * p);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, 3>(mp, tid, j))];
+                inv_pass_t<3>(x, t, q);
+                if (p > 0) {
+                    t = load_tw<LOGN, 3>(mp / 8, mp / 8, tid, itw, itws);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, 3>(mp, tid, j))] = x[j];
+                    __syncthreads();
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                uint64_t v = csub(x[j], q);
+                if (j < 4) v = mul_shoup(v, n_inv, n_inv_s, q);
+                store(pass_index<LOGN, 3>(1u, tid, j), v);
+            }
+            return;
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, Pl::tail_r>(m, tid, j))] = x[j];
         __syncthreads();
@@ -232,7 +283,7 @@ __device__ __forceinline__ void ntt_inverse_cta(uint64_t* sm, uint32_t tid, cons
         const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, 3>(m, tid, j))];
-        inv_pass<LOGN, 3>(x, m, tid, itw, itws, q);
+        inv_pass_t<3>(x, load_tw<LOGN, 3>(m, m, tid, itw, itws), q);
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGN, 3>(m, tid, j))] = x[j];
         __syncthreads();
@@ -241,7 +292,7 @@ __device__ __forceinline__ void ntt_inverse_cta(uint64_t* sm, uint32_t tid, cons
     // folded into itw[1]
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGN, 3>(1u, tid, j))];
-    inv_pass<LOGN, 3>(x, 1u, tid, itw, itws, q);
+    inv_pass_t<3>(x, load_tw<LOGN, 3>(1u, 1u, tid, itw, itws), q);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const uint32_t idx = pass_index<LOGN, 3>(1u, tid, j);

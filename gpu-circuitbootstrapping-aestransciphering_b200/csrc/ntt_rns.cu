@@ -26,97 +26,6 @@
 
 namespace cbs {
 
-// forward pass with an explicit twiddle base: i1 = base + k
-template <int LOGS, int R>
-__device__ __forceinline__ void fwd_pass_b(uint64_t (&x)[8], uint32_t m, uint32_t base, uint32_t tid,
-                                           const uint64_t* __restrict__ tw, const uint64_t* __restrict__ tws,
-                                           uint64_t q) {
-    const uint64_t q2 = q << 1;
-    if (R == 3) {
-        const uint32_t i1 = base + pass_group<LOGS, 3>(m, tid, 0);
-        {
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) ct_bf(x[j], x[j + 4], w, ws, q2, q);
-        }
-        {
-            const uint64_t w0 = __ldg(tw + 2 * i1), w0s = __ldg(tws + 2 * i1);
-            const uint64_t w1 = __ldg(tw + 2 * i1 + 1), w1s = __ldg(tws + 2 * i1 + 1);
-            ct_bf(x[0], x[2], w0, w0s, q2, q);
-            ct_bf(x[1], x[3], w0, w0s, q2, q);
-            ct_bf(x[4], x[6], w1, w1s, q2, q);
-            ct_bf(x[5], x[7], w1, w1s, q2, q);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t ti = 4 * i1 + j;
-            ct_bf(x[2 * j], x[2 * j + 1], __ldg(tw + ti), __ldg(tws + ti), q2, q);
-        }
-    } else if (R == 2) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 2>(m, tid, h);
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-            uint64_t* v = x + 4 * h;
-            ct_bf(v[0], v[2], w, ws, q2, q);
-            ct_bf(v[1], v[3], w, ws, q2, q);
-            ct_bf(v[0], v[1], __ldg(tw + 2 * i1), __ldg(tws + 2 * i1), q2, q);
-            ct_bf(v[2], v[3], __ldg(tw + 2 * i1 + 1), __ldg(tws + 2 * i1 + 1), q2, q);
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 1>(m, tid, h);
-            ct_bf(x[2 * h], x[2 * h + 1], __ldg(tw + i1), __ldg(tws + i1), q2, q);
-        }
-    }
-}
-
-template <int LOGS, int R>
-__device__ __forceinline__ void inv_pass_b(uint64_t (&x)[8], uint32_t m, uint32_t base, uint32_t tid,
-                                           const uint64_t* __restrict__ tw, const uint64_t* __restrict__ tws,
-                                           uint64_t q) {
-    const uint64_t q2 = q << 1;
-    if (R == 3) {
-        const uint32_t i1 = base + pass_group<LOGS, 3>(m, tid, 0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t ti = 4 * i1 + j;
-            gs_bf(x[2 * j], x[2 * j + 1], __ldg(tw + ti), __ldg(tws + ti), q2, q);
-        }
-        {
-            const uint64_t w0 = __ldg(tw + 2 * i1), w0s = __ldg(tws + 2 * i1);
-            const uint64_t w1 = __ldg(tw + 2 * i1 + 1), w1s = __ldg(tws + 2 * i1 + 1);
-            gs_bf(x[0], x[2], w0, w0s, q2, q);
-            gs_bf(x[1], x[3], w0, w0s, q2, q);
-            gs_bf(x[4], x[6], w1, w1s, q2, q);
-            gs_bf(x[5], x[7], w1, w1s, q2, q);
-        }
-        {
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) gs_bf(x[j], x[j + 4], w, ws, q2, q);
-        }
-    } else if (R == 2) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 2>(m, tid, h);
-            uint64_t* v = x + 4 * h;
-            gs_bf(v[0], v[1], __ldg(tw + 2 * i1), __ldg(tws + 2 * i1), q2, q);
-            gs_bf(v[2], v[3], __ldg(tw + 2 * i1 + 1), __ldg(tws + 2 * i1 + 1), q2, q);
-            const uint64_t w = __ldg(tw + i1), ws = __ldg(tws + i1);
-            gs_bf(v[0], v[2], w, ws, q2, q);
-            gs_bf(v[1], v[3], w, ws, q2, q);
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 1>(m, tid, h);
-            gs_bf(x[2 * h], x[2 * h + 1], __ldg(tw + i1), __ldg(tws + i1), q2, q);
-        }
-    }
-}
-
 // 2^LOGS-point forward sub-transform of one group; twb(m) gives the twiddle base of local
 // stage m; load(e), store(e, v) address the group's elements (lazy values)
 template <int LOGS, class TwB, class Load, class Store>
@@ -127,21 +36,21 @@ __device__ __forceinline__ void sub_fwd(uint64_t* sm, uint32_t gt, const uint64_
     uint64_t x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(pass_index<LOGS, 3>(1u, gt, j));
-    fwd_pass_b<LOGS, 3>(x, 1u, twb(1u), gt, tw, tws, q);
+    fwd_pass_t<3>(x, load_tw<LOGS, 3>(1u, twb(1u), gt, tw, tws), q);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
+        const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, 3>(1u << (3 * (p - 1)), gt, j))] = x[j];
         __syncthreads();
-        const uint32_t m = 1u << (3 * p);
         if (p < Pl::P - 1) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, 3>(m, gt, j))];
-            fwd_pass_b<LOGS, 3>(x, m, twb(m), gt, tw, tws, q);
+            fwd_pass_t<3>(x, load_tw<LOGS, 3>(m, twb(m), gt, tw, tws), q);
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, Pl::tail_r>(m, gt, j))];
-            fwd_pass_b<LOGS, Pl::tail_r>(x, m, twb(m), gt, tw, tws, q);
+            fwd_pass_t<Pl::tail_r>(x, load_tw<LOGS, Pl::tail_r>(m, twb(m), gt, tw, tws), q);
         }
     }
     constexpr uint32_t mt = 1u << (3 * (Pl::P - 1));
@@ -158,7 +67,7 @@ __device__ __forceinline__ void sub_inv(uint64_t* sm, uint32_t gt, const uint64_
     uint64_t x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(pass_index<LOGS, Pl::tail_r>(mt, gt, j));
-    inv_pass_b<LOGS, Pl::tail_r>(x, mt, twb(mt), gt, tw, tws, q);
+    inv_pass_t<Pl::tail_r>(x, load_tw<LOGS, Pl::tail_r>(mt, twb(mt), gt, tw, tws), q);
 #pragma unroll
     for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, Pl::tail_r>(mt, gt, j))] = x[j];
     __syncthreads();
@@ -167,7 +76,7 @@ __device__ __forceinline__ void sub_inv(uint64_t* sm, uint32_t gt, const uint64_
         const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, 3>(m, gt, j))];
-        inv_pass_b<LOGS, 3>(x, m, twb(m), gt, tw, tws, q);
+        inv_pass_t<3>(x, load_tw<LOGS, 3>(m, twb(m), gt, tw, tws), q);
         if (p > 0) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, 3>(m, gt, j))] = x[j];
@@ -183,7 +92,7 @@ __device__ __forceinline__ void sub_inv(uint64_t* sm, uint32_t gt, const uint64_
 // FP64-pipe form (primes below 2^50): the exact modular products of fp64_mod.cuh.  Values are
 // signed and lazy: each radix-8 pass first reduces its 8 inputs to |x| <= q/2 + 1, after which
 // three forward stages grow them to at most 2q + 4 and three inverse stages to at most
-// 4q + 8, far inside the exact range.  The twiddles are the same tables converted to doubles;
+// 4q + 8, far inside the exact range.  The twiddles are the same tables as centred doubles;
 // results are the integer path's residues, bit for bit.
 __device__ __forceinline__ void ct_bf_d(double& x, double& y, double w, const DMod& m) {
     const double t = dmulmod(y, w, m);
@@ -197,86 +106,97 @@ __device__ __forceinline__ void gs_bf_d(double& x, double& y, double w, const DM
     y = dmulmod(t, w, m);
 }
 
-// the passes of fwd_pass_b / inv_pass_b with double values and twiddles; inputs reduced first
+// A thread's twiddles of one pass (centred doubles).  The tables are the context's own (16-byte
+// aligned): the pairs and quadruples of a group load as 16-byte words.  They are loaded where the
+// pass begins: loading them before the exchange barrier took the registers of a third CTA per SM,
+// which hides more (forward + inverse of 384 limbs at N = 2^16: 471 us with three CTAs, 519 with
+// early loads and two, 523 with 8-byte loads and two or three).
+//   three stages: [i1] [2 i1, 2 i1 + 1] [4 i1 .. 4 i1 + 3]; two: per set [i1] [2 i1, 2 i1 + 1]; one: [i1] per set
+struct TwD {
+    double w[7];
+};
 template <int LOGS, int R>
-__device__ __forceinline__ void fwd_pass_d(double (&x)[8], uint32_t m, uint32_t base, uint32_t tid,
-                                           const double* __restrict__ tw, const DMod& md) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = dreduce(x[j], md);
+__device__ __forceinline__ TwD load_twd(uint32_t m, uint32_t base, uint32_t tid, const double* __restrict__ tw) {
+    TwD t;
+    auto pair = [&](int at, uint32_t i) {
+        const double2 v = __ldg(reinterpret_cast<const double2*>(tw + i));
+        t.w[at] = v.x;
+        t.w[at + 1] = v.y;
+    };
     if (R == 3) {
         const uint32_t i1 = base + pass_group<LOGS, 3>(m, tid, 0);
-        {
-            const double w = __ldg(tw + i1);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) ct_bf_d(x[j], x[j + 4], w, md);
-        }
-        {
-            const double w0 = __ldg(tw + 2 * i1), w1 = __ldg(tw + 2 * i1 + 1);
-            ct_bf_d(x[0], x[2], w0, md);
-            ct_bf_d(x[1], x[3], w0, md);
-            ct_bf_d(x[4], x[6], w1, md);
-            ct_bf_d(x[5], x[7], w1, md);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ct_bf_d(x[2 * j], x[2 * j + 1], __ldg(tw + 4 * i1 + j), md);
+        t.w[0] = __ldg(tw + i1);
+        pair(1, 2 * i1);
+        pair(3, 4 * i1);
+        pair(5, 4 * i1 + 2);
     } else if (R == 2) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t i1 = base + pass_group<LOGS, 2>(m, tid, h);
-            const double w = __ldg(tw + i1);
-            double* v = x + 4 * h;
-            ct_bf_d(v[0], v[2], w, md);
-            ct_bf_d(v[1], v[3], w, md);
-            ct_bf_d(v[0], v[1], __ldg(tw + 2 * i1), md);
-            ct_bf_d(v[2], v[3], __ldg(tw + 2 * i1 + 1), md);
+            t.w[3 * h] = __ldg(tw + i1);
+            pair(3 * h + 1, 2 * i1);
         }
     } else {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 1>(m, tid, h);
-            ct_bf_d(x[2 * h], x[2 * h + 1], __ldg(tw + i1), md);
+        for (int h = 0; h < 4; ++h) t.w[h] = __ldg(tw + base + pass_group<LOGS, 1>(m, tid, h));
+    }
+    return t;
+}
+
+// the passes of fwd_pass_t / inv_pass_t with double values and twiddles; inputs reduced first
+template <int R>
+__device__ __forceinline__ void fwd_pass_d(double (&x)[8], const TwD& t, const DMod& md) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = dreduce(x[j], md);
+    if (R == 3) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ct_bf_d(x[j], x[j + 4], t.w[0], md);
+        ct_bf_d(x[0], x[2], t.w[1], md);
+        ct_bf_d(x[1], x[3], t.w[1], md);
+        ct_bf_d(x[4], x[6], t.w[2], md);
+        ct_bf_d(x[5], x[7], t.w[2], md);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ct_bf_d(x[2 * j], x[2 * j + 1], t.w[3 + j], md);
+    } else if (R == 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double* v = x + 4 * h;
+            ct_bf_d(v[0], v[2], t.w[3 * h], md);
+            ct_bf_d(v[1], v[3], t.w[3 * h], md);
+            ct_bf_d(v[0], v[1], t.w[3 * h + 1], md);
+            ct_bf_d(v[2], v[3], t.w[3 * h + 2], md);
         }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) ct_bf_d(x[2 * h], x[2 * h + 1], t.w[h], md);
     }
 }
 
-template <int LOGS, int R>
-__device__ __forceinline__ void inv_pass_d(double (&x)[8], uint32_t m, uint32_t base, uint32_t tid,
-                                           const double* __restrict__ tw, const DMod& md) {
+template <int R>
+__device__ __forceinline__ void inv_pass_d(double (&x)[8], const TwD& t, const DMod& md) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = dreduce(x[j], md);
     if (R == 3) {
-        const uint32_t i1 = base + pass_group<LOGS, 3>(m, tid, 0);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) gs_bf_d(x[2 * j], x[2 * j + 1], __ldg(tw + 4 * i1 + j), md);
-        {
-            const double w0 = __ldg(tw + 2 * i1), w1 = __ldg(tw + 2 * i1 + 1);
-            gs_bf_d(x[0], x[2], w0, md);
-            gs_bf_d(x[1], x[3], w0, md);
-            gs_bf_d(x[4], x[6], w1, md);
-            gs_bf_d(x[5], x[7], w1, md);
-        }
-        {
-            const double w = __ldg(tw + i1);
+        for (int j = 0; j < 4; ++j) gs_bf_d(x[2 * j], x[2 * j + 1], t.w[3 + j], md);
+        gs_bf_d(x[0], x[2], t.w[1], md);
+        gs_bf_d(x[1], x[3], t.w[1], md);
+        gs_bf_d(x[4], x[6], t.w[2], md);
+        gs_bf_d(x[5], x[7], t.w[2], md);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) gs_bf_d(x[j], x[j + 4], w, md);
-        }
+        for (int j = 0; j < 4; ++j) gs_bf_d(x[j], x[j + 4], t.w[0], md);
     } else if (R == 2) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 2>(m, tid, h);
             double* v = x + 4 * h;
-            gs_bf_d(v[0], v[1], __ldg(tw + 2 * i1), md);
-            gs_bf_d(v[2], v[3], __ldg(tw + 2 * i1 + 1), md);
-            const double w = __ldg(tw + i1);
-            gs_bf_d(v[0], v[2], w, md);
-            gs_bf_d(v[1], v[3], w, md);
+            gs_bf_d(v[0], v[1], t.w[3 * h + 1], md);
+            gs_bf_d(v[2], v[3], t.w[3 * h + 2], md);
+            gs_bf_d(v[0], v[2], t.w[3 * h], md);
+            gs_bf_d(v[1], v[3], t.w[3 * h], md);
         }
     } else {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const uint32_t i1 = base + pass_group<LOGS, 1>(m, tid, h);
-            gs_bf_d(x[2 * h], x[2 * h + 1], __ldg(tw + i1), md);
-        }
+        for (int h = 0; h < 4; ++h) gs_bf_d(x[2 * h], x[2 * h + 1], t.w[h], md);
     }
 }
 
@@ -290,22 +210,22 @@ __device__ __forceinline__ void sub_fwd_d_hooked(double* sm, uint32_t gt, const 
     double x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(pass_index<LOGS, 3>(1u, gt, j));
-    fwd_pass_d<LOGS, 3>(x, 1u, twb(1u), gt, tw, md);
+    fwd_pass_d<3>(x, load_twd<LOGS, 3>(1u, twb(1u), gt, tw), md);
 #pragma unroll
     for (int p = 1; p < Pl::P; ++p) {
+        const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, 3>(1u << (3 * (p - 1)), gt, j))] = x[j];
         __syncthreads();
         if (p == 1) after_loads();
-        const uint32_t m = 1u << (3 * p);
         if (p < Pl::P - 1) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, 3>(m, gt, j))];
-            fwd_pass_d<LOGS, 3>(x, m, twb(m), gt, tw, md);
+            fwd_pass_d<3>(x, load_twd<LOGS, 3>(m, twb(m), gt, tw), md);
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, Pl::tail_r>(m, gt, j))];
-            fwd_pass_d<LOGS, Pl::tail_r>(x, m, twb(m), gt, tw, md);
+            fwd_pass_d<Pl::tail_r>(x, load_twd<LOGS, Pl::tail_r>(m, twb(m), gt, tw), md);
         }
     }
     constexpr uint32_t mt = 1u << (3 * (Pl::P - 1));
@@ -328,7 +248,7 @@ __device__ __forceinline__ void sub_inv_d(double* sm, uint32_t gt, const double*
     double x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = load(pass_index<LOGS, Pl::tail_r>(mt, gt, j));
-    inv_pass_d<LOGS, Pl::tail_r>(x, mt, twb(mt), gt, tw, md);
+    inv_pass_d<Pl::tail_r>(x, load_twd<LOGS, Pl::tail_r>(mt, twb(mt), gt, tw), md);
 #pragma unroll
     for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, Pl::tail_r>(mt, gt, j))] = x[j];
     __syncthreads();
@@ -337,7 +257,7 @@ __device__ __forceinline__ void sub_inv_d(double* sm, uint32_t gt, const double*
         const uint32_t m = 1u << (3 * p);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = sm[swz(pass_index<LOGS, 3>(m, gt, j))];
-        inv_pass_d<LOGS, 3>(x, m, twb(m), gt, tw, md);
+        inv_pass_d<3>(x, load_twd<LOGS, 3>(m, twb(m), gt, tw), md);
         if (p > 0) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) sm[swz(pass_index<LOGS, 3>(m, gt, j))] = x[j];
@@ -350,6 +270,12 @@ __device__ __forceinline__ void sub_inv_d(double* sm, uint32_t gt, const double*
 
 constexpr int kL2 = 8;            // row stages (rows of 256 words)
 constexpr uint32_t kGroups = 16;  // sub-transforms per CTA
+// CTAs per SM the FP64 column kernels are compiled for: 1536 threads (40 registers), where one CTA
+// leaves room
+template <int L1, bool FP>
+constexpr int col_blocks() {
+    return FP && L1 <= 8 ? 1536 / (16 * (1 << L1) / 8) : 1;
+}
 
 // column groups are padded by one word so the 16 interleaved columns of a warp hit 16
 // different banks
@@ -377,7 +303,7 @@ __device__ __forceinline__ const uint64_t* src_ptr(uint64_t* data, const RnsNttA
 // forward phase 1: columns (2^L1 points each, stride 2^L2), lazy output (FP: signed lazy
 // doubles written in place, read back by the row phase)
 template <int L1, bool FP>
-__global__ void __launch_bounds__(kGroups * (1 << L1) / 8) k_rns_fwd_cols(uint64_t* __restrict__ data,
+__global__ void __launch_bounds__(kGroups * (1 << L1) / 8, col_blocks<L1, FP>()) k_rns_fwd_cols(uint64_t* __restrict__ data,
                                                                          const RnsNttArgs a) {
     constexpr uint32_t ROW = 1u << kL2;
     extern __shared__ uint64_t sm[];
@@ -396,7 +322,7 @@ __global__ void __launch_bounds__(kGroups * (1 << L1) / 8) k_rns_fwd_cols(uint64
         double* dpoly = reinterpret_cast<double*>(poly);
         sub_fwd_d<L1>(
             reinterpret_cast<double*>(sm) + g * col_stride<L1>(), gt, a.twd + prime * N, dmod_of(q),
-            [](uint32_t m) { return m; }, [&](uint32_t e) { return __ull2double_rn(src[e * ROW]); },
+            [](uint32_t m) { return m; }, [&](uint32_t e) { return dfrom_u52(src[e * ROW]); },
             [&](uint32_t e, double v) { dpoly[e * ROW] = v; });
     } else {
         sub_fwd<L1>(
@@ -490,7 +416,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_rns_inv_rows(uint64_t* __restr
         double* drow = reinterpret_cast<double*>(row);
         sub_inv_d<kL2>(
             reinterpret_cast<double*>(sm) + g * ROW, gt, a.itwd + prime * N, dmod_of(q),
-            [&](uint32_t m) { return m * (ROWS + R); }, [&](uint32_t e) { return __ull2double_rn(src[e]); },
+            [&](uint32_t m) { return m * (ROWS + R); }, [&](uint32_t e) { return dfrom_u52(src[e]); },
             [&](uint32_t e, double v, int) { drow[e] = v; });
     } else {
         sub_inv<kL2>(
@@ -501,7 +427,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_rns_inv_rows(uint64_t* __restr
 
 // inverse phase B: columns, n^-1 on the x-half of the last stage, full reduction
 template <int L1, bool FP>
-__global__ void __launch_bounds__(kGroups * (1 << L1) / 8) k_rns_inv_cols(uint64_t* __restrict__ data,
+__global__ void __launch_bounds__(kGroups * (1 << L1) / 8, col_blocks<L1, FP>()) k_rns_inv_cols(uint64_t* __restrict__ data,
                                                                          const RnsNttArgs a) {
     constexpr uint32_t ROW = 1u << kL2;
     extern __shared__ uint64_t sm[];
@@ -520,7 +446,8 @@ __global__ void __launch_bounds__(kGroups * (1 << L1) / 8) k_rns_inv_cols(uint64
     uint64_t* poly = limb_ptr(data, a, limb_flat, L1 + kL2) + colblk * kGroups + g;
     if constexpr (FP) {
         const DMod md = dmod_of(q);
-        const double ninv_d = static_cast<double>(ninv), sc_d = static_cast<double>(sc);
+        // centred: the x-half of the last stage reaches 4q + 8
+        const double ninv_d = static_cast<double>(ninv) - (ninv > q / 2 ? md.q : 0.0), sc_d = static_cast<double>(sc);
         const double* dpoly = reinterpret_cast<const double*>(poly);
         sub_inv_d<L1>(
             reinterpret_cast<double*>(sm) + g * col_stride<L1>(), gt, a.itwd + prime * N, md,
@@ -577,7 +504,7 @@ __device__ __forceinline__ void rows_bulk_store(void* dst, const double* stage) 
 }
 
 template <int L1, int EPI>
-__global__ void __launch_bounds__(kGroups * 32) k_rns_fwd_rows_bulk(uint64_t* __restrict__ data, const RnsNttArgs a) {
+__global__ void __launch_bounds__(kGroups * 32, EPI ? 2 : 3) k_rns_fwd_rows_bulk(uint64_t* __restrict__ data, const RnsNttArgs a) {
     constexpr uint32_t ROW = 1u << kL2, ROWS = 1u << L1;
     extern __shared__ __align__(16) uint64_t sm[];
     double* xsm = reinterpret_cast<double*>(sm);               // exchange [kGroups][ROW]
@@ -649,7 +576,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_rns_fwd_rows_bulk(uint64_t* __
 }
 
 template <int L1>
-__global__ void __launch_bounds__(kGroups * 32) k_rns_inv_rows_bulk(uint64_t* __restrict__ data, const RnsNttArgs a) {
+__global__ void __launch_bounds__(kGroups * 32, 3) k_rns_inv_rows_bulk(uint64_t* __restrict__ data, const RnsNttArgs a) {
     constexpr uint32_t ROW = 1u << kL2, ROWS = 1u << L1;
     extern __shared__ __align__(16) uint64_t sm[];
     double* xsm = reinterpret_cast<double*>(sm);
@@ -671,7 +598,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_rns_inv_rows_bulk(uint64_t* __
     const uint64_t* myu = reinterpret_cast<const uint64_t*>(my);
     sub_inv_d<kL2>(
         xsm + g * ROW, gt, a.itwd + prime * N, dmod_of(q), [&](uint32_t m) { return m * (ROWS + R); },
-        [&](uint32_t e) { return __ull2double_rn(myu[e]); }, [&](uint32_t e, double v, int) { my[e] = v; });
+        [&](uint32_t e) { return dfrom_u52(myu[e]); }, [&](uint32_t e, double v, int) { my[e] = v; });
     rows_bulk_store(blk, stage);
 }
 
@@ -691,14 +618,14 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T) k_rns_small_fwd(uint64_t* __
     uint64_t* dst = limb_ptr(data, a, limb_flat, LOGN);
     const uint64_t* src = src_ptr(data, a, limb_flat, LOGN);
     if (EPI == 0) {
-        ntt_forward_cta<LOGN>(
+        ntt_forward_cta<LOGN, true>(
             sm, threadIdx.x, tw, tws, q, [&](uint32_t i) { return src[i]; },
             [&](int, uint32_t i, uint64_t v) { dst[i] = v; });
     } else {
         const uint64_t* cx = a.epi_cx + poly * a.epi_cx_stride + (static_cast<size_t>(limb) << LOGN);
         uint64_t* out = a.epi_dst + poly * a.epi_dst_stride + (static_cast<size_t>(limb) << LOGN);
         const uint64_t f = a.epi_f[limb], fs = a.epi_fs[limb];
-        ntt_forward_cta<LOGN>(
+        ntt_forward_cta<LOGN, true>(
             sm, threadIdx.x, tw, tws, q, [&](uint32_t i) { return src[i]; },
             [&](int, uint32_t i, uint64_t v) {
                 uint64_t r = mul_shoup(sub_mod(cx[i], v, q), f, fs, q);
@@ -719,7 +646,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN>::T) k_rns_small_inv(uint64_t* __
     const uint64_t sc = a.scale ? a.scale[limb] : 0, scs = a.scale ? a.scale_s[limb] : 0;
     uint64_t* dst = limb_ptr(data, a, limb_flat, LOGN);
     const uint64_t* src = src_ptr(data, a, limb_flat, LOGN);
-    ntt_inverse_cta<LOGN>(
+    ntt_inverse_cta<LOGN, true>(
         sm, threadIdx.x, a.itw + prime * N, a.itws + prime * N, a.n_inv[prime], a.n_inv_s[prime], q,
         [&](int, uint32_t i) { return src[i]; },
         [&](uint32_t i, uint64_t v) { dst[i] = sc ? mul_shoup(v, sc, scs, q) : v; });

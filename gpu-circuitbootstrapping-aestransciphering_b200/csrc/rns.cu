@@ -116,28 +116,33 @@ __global__ void __launch_bounds__(kThreads) k_modup_bconv(const uint64_t* __rest
 }
 
 // the same base conversion on the FP64 pipe (every prime below 2^50, fp64_mod.cuh): products
-// reduced exactly to |r| <= 0.875 q, partial sums folded every 8 terms; same residues
+// reduced exactly to |r| <= 0.875 q, partial sums folded every 8 terms; same residues.  AMAX: the
+// context's alpha rounded up to 1, 2, 4, 8 or 16, so the term loops carry no idle terms and the
+// digit's residues stay in 2 AMAX registers; the conversion constants are staged as doubles, not
+// converted once per term.  FP64 issue and its writes share the time: 12 digits of 2 into 26 limbs,
+// N = 2^16, 4 ciphertexts (655 MB): 291 us with 16-term loops and integer constants, 169 us here.
+template <int AMAX>
 __global__ void __launch_bounds__(kThreads) k_modup_bconv_d(const uint64_t* __restrict__ coef,
                                                             const uint64_t* __restrict__ c2, uint64_t* __restrict__ t,
                                                             const ModupArgs a) {
-    extern __shared__ uint64_t s_qhat[];
+    extern __shared__ double s_qhat_d[];
     const uint32_t b = blockIdx.y, ct = blockIdx.z;
     const uint32_t start = a.alpha * b;
     const uint32_t cnt = (b == a.beta - 1) ? a.ql - a.alpha * (a.beta - 1) : a.alpha;
     const uint32_t ncompl = a.qlp - cnt;
     const uint64_t* qh = a.qhat + static_cast<size_t>(b) * a.qlp * a.alpha;
-    for (uint32_t i = threadIdx.x; i < ncompl * a.alpha; i += blockDim.x) s_qhat[i] = qh[i];
+    for (uint32_t i = threadIdx.x; i < ncompl * a.alpha; i += blockDim.x) s_qhat_d[i] = dfrom_u52(qh[i]);
     __syncthreads();
     const size_t N = size_t(1) << a.log_n;
     const size_t c = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t* ci = coef + static_cast<size_t>(ct) * a.ql * N + start * N + c;
     const uint64_t* c2i = c2 + static_cast<size_t>(ct) * a.ql * N + start * N + c;
     uint64_t* tb = t + (static_cast<size_t>(ct) * a.beta + b) * a.qlp * N + c;
-    double y[kMaxAlpha];
+    double y[AMAX];
 #pragma unroll
-    for (uint32_t i = 0; i < kMaxAlpha; ++i) {
+    for (uint32_t i = 0; i < AMAX; ++i) {
         if (i < cnt) {
-            y[i] = __ull2double_rn(ci[i * N]);
+            y[i] = dfrom_u52(ci[i * N]);
             tb[(start + i) * N] = c2i[i * N];
         }
     }
@@ -145,14 +150,14 @@ __global__ void __launch_bounds__(kThreads) k_modup_bconv_d(const uint64_t* __re
     const uint32_t* prime = a.out_prime + static_cast<size_t>(b) * a.qlp;
     for (uint32_t k = 0; k < ncompl; ++k) {
         const uint32_t pk = __ldg(prime + k);
-        const DMod md{static_cast<double>(__ldg(a.q + pk)), __ldg(a.qinv + pk)};
-        const uint64_t* w = s_qhat + k * a.alpha;
+        const DMod md{dfrom_u52(__ldg(a.q + pk)), __ldg(a.qinv + pk)};
+        const double* w = s_qhat_d + k * a.alpha;
         double acc = 0.0;
 #pragma unroll
-        for (uint32_t i = 0; i < kMaxAlpha; ++i) {
+        for (uint32_t i = 0; i < AMAX; ++i) {
             if (i < cnt) {
                 if (i && (i & 7u) == 0) acc = dreduce(acc, md);
-                acc = __dadd_rn(acc, dmulmod(y[i], __ull2double_rn(w[i]), md));
+                acc = __dadd_rn(acc, dmulmod(y[i], w[i], md));
             }
         }
         tb[static_cast<size_t>(__ldg(slot + k)) * N] = dto_residue(acc, md);
@@ -228,8 +233,8 @@ __global__ void __launch_bounds__(kThreads) k_ks_inner_d(const uint64_t* __restr
     const DMod md = dmod_of(__ldg(a.q + pr));
     uint32_t since = 0;
     for (uint32_t b = 0; b < a.beta; ++b) {
-        const double e0 = __ull2double_rn(__ldg(evk.p[b] + static_cast<size_t>(pr) * N + c));
-        const double e1 = __ull2double_rn(__ldg(evk.p[b] + (static_cast<size_t>(a.qp) + pr) * N + c));
+        const double e0 = dfrom_u52(__ldg(evk.p[b] + static_cast<size_t>(pr) * N + c));
+        const double e1 = dfrom_u52(__ldg(evk.p[b] + (static_cast<size_t>(a.qp) + pr) * N + c));
         const uint64_t* tb = t + (static_cast<size_t>(b) * a.qlp + l) * N + c;
         if (since == 8) {
 #pragma unroll
@@ -242,7 +247,7 @@ __global__ void __launch_bounds__(kThreads) k_ks_inner_d(const uint64_t* __restr
 #pragma unroll
         for (int j = 0; j < CT; ++j) {
             if (ct0 + j < a.count) {
-                const double x = __ull2double_rn(tb[(ct0 + j) * tstride]);
+                const double x = dfrom_u52(tb[(ct0 + j) * tstride]);
                 acc0[j] = __dadd_rn(acc0[j], dmulmod(x, e0, md));
                 acc1[j] = __dadd_rn(acc1[j], dmulmod(x, e1, md));
             }
@@ -255,6 +260,70 @@ __global__ void __launch_bounds__(kThreads) k_ks_inner_d(const uint64_t* __restr
             uint64_t* o = cx + (static_cast<size_t>(ct0 + j) * 2 * a.qlp + l) * N + c;
             o[0] = dto_residue(acc0[j], md);
             o[static_cast<size_t>(a.qlp) * N] = dto_residue(acc1[j], md);
+        }
+    }
+}
+
+// The same with two adjacent coefficients per thread, in 16-byte loads and stores.  Memory bounds
+// it (12 digits, 26 limbs, N = 2^16, 4 ciphertexts: 0.98 GB, 149 us at the copy rate); with one
+// coefficient per thread too few bytes were in flight: 337 us, here 176 us (unrolling the digits of
+// that form by 2 or 4: 374 and 371 us).
+template <int CT>
+__global__ void __launch_bounds__(kThreads) k_ks_inner_d2(const uint64_t* __restrict__ t, const EvkPtrs evk,
+                                                          uint64_t* __restrict__ cx, const InnerArgs a) {
+    const size_t N = size_t(1) << a.log_n;
+    const size_t idx = 2 * (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x);  // l * N + c
+    const uint32_t l = static_cast<uint32_t>(idx >> a.log_n);
+    if (l >= a.qlp) return;
+    const size_t c = idx & (N - 1);
+    const uint32_t pr = __ldg(a.prime + l);
+    const uint32_t ct0 = blockIdx.y * CT;
+    double acc[CT][2][2];  // [ciphertext][component][coefficient]
+#pragma unroll
+    for (int j = 0; j < CT; ++j) acc[j][0][0] = acc[j][0][1] = acc[j][1][0] = acc[j][1][1] = 0.0;
+    const size_t tstride = static_cast<size_t>(a.beta) * a.qlp * N;  // per ciphertext
+    const DMod md = dmod_of(__ldg(a.q + pr));
+    auto get = [](const uint64_t* p) { return __ldg(reinterpret_cast<const ulonglong2*>(p)); };
+    uint32_t since = 0;
+    for (uint32_t b = 0; b < a.beta; ++b) {
+        const ulonglong2 e0 = get(evk.p[b] + static_cast<size_t>(pr) * N + c);
+        const ulonglong2 e1 = get(evk.p[b] + (static_cast<size_t>(a.qp) + pr) * N + c);
+        const uint64_t* tb = t + (static_cast<size_t>(b) * a.qlp + l) * N + c;
+        ulonglong2 x[CT];
+#pragma unroll
+        for (int j = 0; j < CT; ++j)
+            if (ct0 + j < a.count) x[j] = get(tb + (ct0 + j) * tstride);
+        if (since == 8) {
+#pragma unroll
+            for (int j = 0; j < CT; ++j)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    acc[j][k][0] = dreduce(acc[j][k][0], md);
+                    acc[j][k][1] = dreduce(acc[j][k][1], md);
+                }
+            since = 0;
+        }
+        const double e[2][2] = {{dfrom_u52(e0.x), dfrom_u52(e0.y)}, {dfrom_u52(e1.x), dfrom_u52(e1.y)}};
+#pragma unroll
+        for (int j = 0; j < CT; ++j) {
+            if (ct0 + j < a.count) {
+                const double v[2] = {dfrom_u52(x[j].x), dfrom_u52(x[j].y)};
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int z = 0; z < 2; ++z) acc[j][k][z] = __dadd_rn(acc[j][k][z], dmulmod(v[z], e[k][z], md));
+            }
+        }
+        ++since;
+    }
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+        if (ct0 + j < a.count) {
+            uint64_t* o = cx + (static_cast<size_t>(ct0 + j) * 2 * a.qlp + l) * N + c;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                *reinterpret_cast<ulonglong2*>(o + k * static_cast<size_t>(a.qlp) * N) =
+                    make_ulonglong2(dto_residue(acc[j][k][0], md), dto_residue(acc[j][k][1], md));
         }
     }
 }
@@ -285,30 +354,31 @@ __global__ void __launch_bounds__(kThreads) k_moddown_bconv(const uint64_t* __re
     }
 }
 
-// the same on the FP64 pipe (every prime below 2^50, fp64_mod.cuh); same residues
+// the same on the FP64 pipe (every prime below 2^50, fp64_mod.cuh); same residues; AMAX as above
+template <int AMAX>
 __global__ void __launch_bounds__(kThreads) k_moddown_bconv_d(const uint64_t* __restrict__ cx,
                                                               uint64_t* __restrict__ delta, const ModdownArgs a) {
-    extern __shared__ uint64_t s_phat[];
-    for (uint32_t i = threadIdx.x; i < a.ql * a.alpha; i += blockDim.x) s_phat[i] = a.phat[i];
+    extern __shared__ double s_phat_d[];
+    for (uint32_t i = threadIdx.x; i < a.ql * a.alpha; i += blockDim.x) s_phat_d[i] = dfrom_u52(a.phat[i]);
     __syncthreads();
     const size_t N = size_t(1) << a.log_n;
     const size_t c = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t poly = blockIdx.y;
     const uint64_t* src = cx + (static_cast<size_t>(poly) * a.qlp + a.ql) * N + c;
-    double y[kMaxAlpha];
+    double y[AMAX];
 #pragma unroll
-    for (uint32_t j = 0; j < kMaxAlpha; ++j)
-        if (j < a.alpha) y[j] = __ull2double_rn(src[j * N]);
+    for (uint32_t j = 0; j < AMAX; ++j)
+        if (j < a.alpha) y[j] = dfrom_u52(src[j * N]);
     uint64_t* dst = delta + static_cast<size_t>(poly) * a.ql * N + c;
     for (uint32_t i = 0; i < a.ql; ++i) {
-        const DMod md{static_cast<double>(__ldg(a.q + i)), __ldg(a.qinv + i)};
-        const uint64_t* w = s_phat + i * a.alpha;
+        const DMod md{dfrom_u52(__ldg(a.q + i)), __ldg(a.qinv + i)};
+        const double* w = s_phat_d + i * a.alpha;
         double acc = 0.0;
 #pragma unroll
-        for (uint32_t j = 0; j < kMaxAlpha; ++j) {
+        for (uint32_t j = 0; j < AMAX; ++j) {
             if (j < a.alpha) {
                 if (j && (j & 7u) == 0) acc = dreduce(acc, md);
-                acc = __dadd_rn(acc, dmulmod(y[j], __ull2double_rn(w[j]), md));
+                acc = __dadd_rn(acc, dmulmod(y[j], w[j], md));
             }
         }
         dst[i * N] = dto_residue(acc, md);
@@ -464,7 +534,12 @@ cbs_status run_modup(cbs_rns_context* c, cbs::RnsLevel* lv, uint64_t* d_t, const
     const size_t smem = static_cast<size_t>(lv->qlp) * lv->alpha * sizeof(uint64_t);
     if (c->d_qinv.p) {
         m.qinv = c->d_qinv.p;
-        cbs::k_modup_bconv_d<<<grid, cbs::kThreads, smem, s>>>(c->s_coef.p, d_c2, d_t, m);
+        const auto kernel = lv->alpha == 1   ? cbs::k_modup_bconv_d<1>
+                            : lv->alpha == 2 ? cbs::k_modup_bconv_d<2>
+                            : lv->alpha <= 4 ? cbs::k_modup_bconv_d<4>
+                            : lv->alpha <= 8 ? cbs::k_modup_bconv_d<8>
+                                             : cbs::k_modup_bconv_d<16>;
+        kernel<<<grid, cbs::kThreads, smem, s>>>(c->s_coef.p, d_c2, d_t, m);
     } else {
         cbs::k_modup_bconv<<<grid, cbs::kThreads, smem, s>>>(c->s_coef.p, d_c2, d_t, m);
     }
@@ -490,7 +565,13 @@ cbs_status run_inner(cbs_rns_context* c, cbs::RnsLevel* lv, uint64_t* d_cx, cons
     cbs::InnerArgs a{lv->ip_prime.p, c->d_q.p, c->d_r0.p, c->d_r1.p, c->log_n, lv->qlp, c->size_qp,
                      lv->beta, count, c->red_k};
     const dim3 grid(static_cast<unsigned>(static_cast<size_t>(lv->qlp) * c->n / cbs::kThreads), (count + CT - 1) / CT);
-    if (c->d_twd.p) cbs::k_ks_inner_d<CT><<<grid, cbs::kThreads, 0, s>>>(d_t, e, d_cx, a);
+    // pairs want every caller's pointer on 16 bytes (strides are multiples of N words)
+    uintptr_t bits = reinterpret_cast<uintptr_t>(d_t) | reinterpret_cast<uintptr_t>(d_cx);
+    for (uint32_t b = 0; b < lv->beta; ++b) bits |= reinterpret_cast<uintptr_t>(h_evks[b]);
+    const dim3 half(grid.x / 2, grid.y);
+    if (c->d_twd.p && bits % 16 == 0 && c->n % (2 * cbs::kThreads) == 0)
+        cbs::k_ks_inner_d2<CT><<<half, cbs::kThreads, 0, s>>>(d_t, e, d_cx, a);
+    else if (c->d_twd.p) cbs::k_ks_inner_d<CT><<<grid, cbs::kThreads, 0, s>>>(d_t, e, d_cx, a);
     else cbs::k_ks_inner<CT><<<grid, cbs::kThreads, 0, s>>>(d_t, e, d_cx, a);
     CBS_LAUNCH_CHECK();
     return CBS_OK;
@@ -517,7 +598,12 @@ cbs_status run_moddown(cbs_rns_context* c, cbs::RnsLevel* lv, uint64_t* d_ct, ui
     const size_t md_smem = static_cast<size_t>(lv->ql) * lv->alpha * sizeof(uint64_t);
     if (c->d_qinv.p) {
         m.qinv = c->d_qinv.p;
-        cbs::k_moddown_bconv_d<<<grid, cbs::kThreads, md_smem, s>>>(d_cx, c->s_delta.p, m);
+        const auto kernel = lv->alpha == 1   ? cbs::k_moddown_bconv_d<1>
+                            : lv->alpha == 2 ? cbs::k_moddown_bconv_d<2>
+                            : lv->alpha <= 4 ? cbs::k_moddown_bconv_d<4>
+                            : lv->alpha <= 8 ? cbs::k_moddown_bconv_d<8>
+                                             : cbs::k_moddown_bconv_d<16>;
+        kernel<<<grid, cbs::kThreads, md_smem, s>>>(d_cx, c->s_delta.p, m);
     } else {
         cbs::k_moddown_bconv<<<grid, cbs::kThreads, md_smem, s>>>(d_cx, c->s_delta.p, m);
     }
@@ -632,7 +718,16 @@ cbs_status cbs_rns_context_create(uint32_t poly_degree, const uint64_t* h_q, uin
     CBS_CUDA_TRY(cudaMemset(c->d_fault.p, 0, sizeof(uint32_t)));
     if (qmax < (uint64_t(1) << 50)) {
         // exact doubles of the twiddles for the FP64-pipe transforms
-        std::vector<double> twd(tw.begin(), tw.end()), itwd(itw.begin(), itw.end()), qinv(L);
+        // centred: |w| <= q / 2 keeps every quotient of the transforms below 2^51 (fp64_mod.cuh)
+        std::vector<double> twd(tw.size()), itwd(itw.size()), qinv(L);
+        auto centred = [&](uint64_t w, size_t i) {
+            const uint64_t q = primes[i / N];
+            return w > q / 2 ? -static_cast<double>(q - w) : static_cast<double>(w);
+        };
+        for (size_t i = 0; i < tw.size(); ++i) {
+            twd[i] = centred(tw[i], i);
+            itwd[i] = centred(itw[i], i);
+        }
         for (size_t i = 0; i < L; ++i) qinv[i] = 1.0 / static_cast<double>(primes[i]);
         CBS_CUDA_TRY(upload_sync(c->d_twd, twd));
         CBS_CUDA_TRY(upload_sync(c->d_itwd, itwd));

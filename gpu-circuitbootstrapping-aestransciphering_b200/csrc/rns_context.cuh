@@ -39,7 +39,7 @@ struct cbs_rns_context {
     std::vector<uint64_t> primes;  // Q chain then P
     std::vector<cbs::host::NttTables> tabs;
     cbs::DevBuf<uint64_t> d_tw, d_tws, d_itw, d_itws, d_q, d_ninv, d_ninv_s, d_r0, d_r1;
-    cbs::DevBuf<double> d_twd, d_itwd;  // tw / itw as doubles when every prime is below 2^50
+    cbs::DevBuf<double> d_twd, d_itwd;  // tw / itw as centred doubles when every prime is below 2^50
     cbs::DevBuf<double> d_qinv;         // fl(1 / q) per prime, likewise
     cbs::DevBuf<uint32_t> d_fault;      // device fault word (CBS_FAULT_* bits)
     cbs::DevBuf<cbs_dmodulus> d_mod;
