@@ -328,9 +328,12 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
 
     chunks = -(-blocks // 256)
     # per round: blind rotation, HomTrace+SchemeSwitch, 8 CMux levels, word assembly and
-    # extraction (+ one inverse NTT of the words on the NTT backend); + state init per chunk
-    # (the split backend adds one forward NTT of the MV outputs after its blind rotation)
-    launches_per_step = chunks * (1 + ROUNDS * {"fft64": 12, "ntt": 13, "fft64-split": 14}[args.backend])
+    # extraction (3 launches; + one inverse NTT of the words on the NTT backend); + state init per
+    # chunk (the split backend adds one forward NTT of the MV outputs after its blind rotation)
+    per_round = {"fft64": 14, "ntt": 15, "fft64-split": 16}[args.backend]
+    if args.backend == "fft64" and args.multibit == 2 and (tuned or args.schedule == 0):
+        per_round += br_launches(128 * blocks // chunks, 2) - 1  # + the last wave's remainder
+    launches_per_step = chunks * (1 + ROUNDS * per_round)
     result = {
         "metric": METRICS[args.backend],
         "value": rep.whole_job_rate(world, blocks, ms_per_step),
@@ -684,7 +687,9 @@ def run_gate(args, rank: int, world: int, local_rank: int) -> None:
                       "fft_mode": args.fft_mode,
                       "gadget": f"2^{p.bg_bits}x{p.levels}", "ks": f"2^{p.ks_base_bits}x{p.ks_levels}",
                       "l2": "keys (62 MB spectra + 62 MB KSK) stay L2/HBM resident; no flush"},
-           "us_per_gate": ms * 1e3 / count, "correct_gates": ok, "gpu_launches": args.steps * 2,
+           "us_per_gate": ms * 1e3 / count, "correct_gates": ok,
+           # blind rotation, then initial words and tensor-core product of the key switch
+           "gpu_launches": args.steps * (2 + (br_launches(count, 4) if args.multibit == 2 else 1)),
            "e2e": {"value": world * count / (e2e_ms * 1e-3), "unit": "gates/s",
                    "h2d_bytes_per_step": 2 * count * (p.n + 1) * 4, "d2h_bytes_per_step": count * (p.n + 1) * 4},
            "roofline": {"kernel": f"{fm['kernel']} + k_gate_keyswitch", "bound": "hbm", "achieved": gbs,
@@ -786,9 +791,9 @@ def run_ragged(args, rank: int, world: int, local_rank: int) -> None:
                       "br_multibit": args.multibit, "fft_mode": args.fft_mode,
                       "per_set": [sum(r[4] for r in reqs[0]), sum(r[4] for r in reqs[1])],
                       "l2": "keys of both sets (2 x ~125 MB) do not fit L2 together; no flush"},
-           "correct": ok, "gpu_launches": args.steps * 4,
+           "correct": ok, "gpu_launches": args.steps * 6,
            "per_request_launches": {"ms_per_step": per_ms, "value": world * total / (per_ms * 1e-3),
-                                    "launches_per_step": 2 * len(bufs), "ragged_speedup": per_ms / ms},
+                                    "launches_per_step": 3 * len(bufs), "ragged_speedup": per_ms / ms},
            "autotune": {"chosen_grid_ctas": list(best), "per_set": tune,
                         "note": "cbs_gate_ragged_autotune: one timed launch per candidate grid and set"},
            "clocks": clk.summary()}
@@ -866,6 +871,15 @@ def run_tcb(args, rank: int, world: int, local_rank: int) -> None:
 def mb_keys(mb: int) -> int:
     """Grouped keys per group: 2^mb - 1 subsets, 8 for the staged mb = 4 (3 + 1)."""
     return 8 if mb == 4 else (1 << mb) - 1
+
+
+def br_launches(items: int, per_sm: int) -> int:
+    """Launches of a grouped (mb = 2) blind rotation: what the last wave of the throughput form
+    (per_sm ciphertexts per SM) leaves over runs in the small-batch form when it is at most half a wave."""
+    import torch
+    wave = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    rest = items % wave
+    return 2 if 0 < rest <= wave // 2 and rest < items else 1
 
 
 def br_key_bytes(p, mb: int) -> int:

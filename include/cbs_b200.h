@@ -241,13 +241,15 @@ cbs_status cbs_lmkcdey_auto_maps_host(uint32_t N, uint32_t num_auto_keys, uint32
  * ciphertext; the reference runs one ciphertext per call from the host. */
 cbs_status cbs_lmkcdey_eval_acc_batch_device(cbs_context *ctx, const uint32_t *a_neg, uint32_t a_stride, uint64_t *acc,
                                              uint32_t batch, cbs_stream_t stream);
-/* Schedule of the grouped FFT blind rotation with a two-digit gadget: CBS_BR_SCHEDULE_LOCKSTEP
- * transforms both digits of a polynomial together (interleaved butterflies, shared barriers),
- * CBS_BR_SCHEDULE_DIGITWISE one after the other, CBS_BR_SCHEDULE_PAIRED runs two ciphertexts per
- * CTA (mb = 2, N = 2048; 16 warps per SM, work split by output column);
- * CBS_BR_SCHEDULE_AUTO (default) takes the autotuner's cached choice for this GPU and parameter
- * set, else paired where it applies (mb = 2, N = 2048), else lockstep.  Results differ only by
- * FP64 rounding (all within the phase-error bound).  No reference counterpart. */
+/* Schedule of the grouped FFT blind rotation: CBS_BR_SCHEDULE_LOCKSTEP
+ * transforms both digits of a polynomial together (two-digit gadget; interleaved butterflies,
+ * shared barriers), CBS_BR_SCHEDULE_DIGITWISE one after the other, CBS_BR_SCHEDULE_PAIRED runs two
+ * ciphertexts per CTA (mb = 2, N = 2048, two or three digits; 16 warps per SM, every key load
+ * shared); CBS_BR_SCHEDULE_AUTO (default) takes the autotuner's cached choice for this GPU and
+ * parameter set, else paired where it applies, else lockstep, and at mb = 2 runs a batch below one
+ * ciphertext per SM, or a last wave at most half full, with one ciphertext per CTA of 512 threads or
+ * per cluster of two.  Results differ only by FP64 rounding (all within the phase-error bound).  No
+ * reference counterpart. */
 enum { CBS_BR_SCHEDULE_AUTO = 0, CBS_BR_SCHEDULE_DIGITWISE = 1, CBS_BR_SCHEDULE_LOCKSTEP = 2,
        CBS_BR_SCHEDULE_PAIRED = 3 };
 cbs_status cbs_context_set_br_schedule(cbs_context *ctx, uint32_t schedule);
